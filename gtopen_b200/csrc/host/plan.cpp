@@ -637,11 +637,13 @@ Plan build_plan(const Spot& sp, bool use_iso, int fuse_mode, int shard, int nsha
         if (!visited[nd] || t.kind[nd] != kAction) continue;
         int a = t.player[nd];
         uint64_t len = (uint64_t)t.nchild[nd] * P.nh[a];
+        // padded to whole groups of four hands: the vector kernels read and write groups
+        const uint64_t padded = (uint64_t)t.nchild[nd] * ((P.nh[a] + 3) / 4 * 4);
         P.node_sidx[nd] = (int32_t)P.n_anodes[a];
         P.anode_id[a].push_back(nd);
         P.anode_off[a].push_back(P.arena_len[a]);
         P.n_anodes[a]++;
-        P.arena_len[a] += (len + kArenaAlign - 1) / kArenaAlign * kArenaAlign;
+        P.arena_len[a] += (padded + kArenaAlign - 1) / kArenaAlign * kArenaAlign;
         P.visited_action_elems[a] += len;
     }
     parallel_for((P.act.size() + 65535) / 65536, [&](size_t c) {

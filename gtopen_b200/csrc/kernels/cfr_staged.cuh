@@ -22,21 +22,7 @@ namespace gtob {
 
 constexpr int kSThreads = 128;
 constexpr int kSWarps = kSThreads / 32;
-constexpr int kSKA = 4;                                // staged kernels take nodes with at most 4 actions
 constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s
-
-// One action node as the staged kernels read it: everything its copies need
-// in one 80-byte record (one load round trip per node).
-struct alignas(16) SNode {
-    uint64_t aoff;             // arena offset (elements) in the actor's arena
-    uint32_t cslot, rslot, oslot, sidx;
-    uint32_t cs[kSKA];         // child cfv slots (kNoSlot: the fold child)
-    uint32_t rs[kSKA];         // child reach slots of the actor (down sweep; kNoSlot: none)
-    uint32_t actor, na, fk;    // fk: the fold child's index, kNoSlot if none
-    uint32_t folder;           // the folding player of the fold child
-    float twin, tlose;         // fold payoffs
-};
-static_assert(sizeof(SNode) == 80, "SNode layout");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -348,31 +334,6 @@ struct SLayout {
     __host__ __device__ unsigned cv() const { return o_cv; }
 };
 
-// The two quantised arena formats: 16-bit (store.rs: i16 regrets, u16
-// strategy sums) and FP8 E4M3 (both signed 8-bit), each with a per-node scale
-// = the block's max magnitude, stored as value * (kR or kS) / scale.
-template <int FMT>
-struct QT {
-    using R = int16_t;
-    using S = uint16_t;
-    static constexpr float kR = 32767.0f, kS = 65535.0f;
-    __device__ static float dr(R q) { return (float)q; }
-    __device__ static float ds(S q) { return (float)q; }
-    __device__ static R er(float x) { return sat_i16(x); }
-    __device__ static S es(float x) { return sat_u16(x); }
-};
-template <>
-struct QT<kDevFP8> {
-    using R = uint8_t;
-    using S = uint8_t;
-    static constexpr float kR = 448.0f, kS = 448.0f;
-    __device__ static float dr(R q) { return e4m3_to_f32(q); }
-    __device__ static float ds(S q) { return e4m3_to_f32(q); }
-    __device__ static R er(float x) { return f32_to_e4m3(x); }
-    __device__ static S es(float x) { return f32_to_e4m3(x); }
-};
-__host__ __device__ constexpr int fmt_bytes(int fmt) { return fmt == kDevF32 ? 4 : fmt == kDevFP8 ? 1 : 2; }
-
 // Down sweep, one node per CTA: staged sigma source and parent reach; child
 // reach vectors written with coalesced stores (cfr.rs:469-531 push-down).
 template <int FMT, int NA, int NT = kSThreads>
@@ -426,19 +387,6 @@ __device__ __forceinline__ void ks_down_node(const Dev& d, const Arenas& ar, con
             if (k < na && it.rs[k] != kNoSlot) d.reach[a][(size_t)it.rs[k] * d.rstr[a] + i] = p * sig[k];
     }
 }
-template <int FMT>
-__global__ void __launch_bounds__(kSThreads) ks_down(Dev d, Arenas ar, const SNode* nodes, int mode) {
-    extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ int s_flag;
-    const SNode it = nodes[blockIdx.x];
-    switch (it.na) {  // uniform per CTA: one specialised body per action count
-        case 1: ks_down_node<FMT, 1>(d, ar, it, mode, sm, s_flag); break;
-        case 2: ks_down_node<FMT, 2>(d, ar, it, mode, sm, s_flag); break;
-        case 3: ks_down_node<FMT, 3>(d, ar, it, mode, sm, s_flag); break;
-        default: ks_down_node<FMT, 4>(d, ar, it, mode, sm, s_flag); break;
-    }
-}
-
 // Up sweep, one node per CTA (cfr.rs:469-531 pull-up, 297-409 update;
 // best_response.rs:69-121, 185-219 for EVAL = 1 with mode 0 BR / 1 average).
 // The node's fold child, if any, is evaluated here from the staged opponent
@@ -764,21 +712,6 @@ __device__ __forceinline__ void ks_up_node(const Dev& d, const Arenas& ar, const
                                            b_str, b_pred, cv, vstride, rp, out, false, s_red);
 #undef CHILD_V
 }
-// MINE: the launch's nodes are the traverser's (the update), else the
-// opponent's (sum of children); a launch never mixes the two.
-template <int FMT, int EVAL, bool MINE>
-__global__ void __launch_bounds__(kSThreads) ks_up(Dev d, Arenas ar, const SNode* nodes, int p, int mode) {
-    extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ UpShared us;
-    const SNode it = nodes[blockIdx.x];
-    switch (it.na) {  // uniform per CTA: one specialised body per action count
-        case 1: ks_up_node<FMT, EVAL, 1, MINE>(d, ar, it, p, mode, sm, us); break;
-        case 2: ks_up_node<FMT, EVAL, 2, MINE>(d, ar, it, p, mode, sm, us); break;
-        case 3: ks_up_node<FMT, EVAL, 3, MINE>(d, ar, it, p, mode, sm, us); break;
-        default: ks_up_node<FMT, EVAL, 4, MINE>(d, ar, it, p, mode, sm, us); break;
-    }
-}
-
 // ------------------------------------------------- batched showdowns
 // One CTA per batch of up to kShowBatch showdowns of one level that share a
 // river slot (game.rs:501-577 with the plan's rank tables).  The slot's

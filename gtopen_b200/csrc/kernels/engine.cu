@@ -39,6 +39,7 @@
 #include "cfr_staged.cuh"
 #include "cfr_river.cuh"
 #include "cfr_batch.cuh"
+#include "cfr_vec.hpp"
 #include "engine.hpp"
 
 namespace gtob {
@@ -98,7 +99,8 @@ struct EngineImpl {
     bool wide = false;  // some node has more than 8 actions: use the 32-wide kernels
     bool term64 = false;  // terminal sums in f64 (plain engine, or fused on request)
     bool warp = false;    // warp-per-node action kernels, fold children in place
-    bool staged = false;  // staged (bulk-copy) node kernels, fold children in place
+    bool staged = false;  // staged (bulk-copy) node records: nodes of at most 4 actions
+    bool vec = false;     // vector node kernels in the level sweeps: nodes of at most 8 actions
     bool reach_valid = false;  // reach slots hold the current strategies' reach (see prime)
     uint32_t iteration = 0;
     cudaStream_t stream = nullptr;
@@ -126,6 +128,11 @@ struct EngineImpl {
     size_t warp_smem = 0;    // warp up-action dynamic smem (one staged reach per warp)
     size_t st_mine_smem = 0, st_opp_smem = 0, st_down_smem = 0;  // staged kernels
     SNode* snodes = nullptr;                   // staged node records (same order as act)
+    SNodeT<kVKA>* wnodes = nullptr;            // the wide records instead, with nodes of 5 to 8 actions
+    // records [s.start, s.start + s.count) for the vector kernels
+    VecNodes vnodes(const Span& s) const {
+        return {snodes ? (const void*)(snodes + s.start) : (const void*)(wnodes + s.start), s.count, !snodes};
+    }
     size_t show_pair_smem = 0;                                    // batched showdowns
     // river programs (cfr_river.cuh): each river betting round solved by one
     // CTA; the level sweeps then cover only the nodes outside river rounds
@@ -308,9 +315,7 @@ struct EngineImpl {
     }
     template <int FMT, int KA>
     void down_action(const Span& sa, int mode) {
-        if (staged) {
-            ks_down<FMT><<<sa.count, kSThreads, st_down_smem, stream>>>(d, ar, snodes + sa.start, mode);
-        } else if (warp) {
+        if (warp) {
             const unsigned grid = (sa.count + kWarps - 1) / kWarps;
             kw_down_action<FMT, KA><<<grid, kThreads, 0, stream>>>(d, ar, act + sa.start, (int)sa.count, mode);
         } else {
@@ -329,42 +334,17 @@ struct EngineImpl {
         set_smem((const void*)kw_up_action<FMT, 0, KA>, bytes);
         set_smem((const void*)kw_up_action<FMT, 1, KA>, bytes);
     }
-    template <int FMT, bool MINE>
-    void staged_up(const Span& s, int p, int eval) {
-        if (!s.count) return;
-        const SNode* it = snodes + s.start;
-        const size_t sm = MINE ? st_mine_smem : st_opp_smem;
-        if (eval < 0) ks_up<FMT, 0, MINE><<<s.count, kSThreads, sm, stream>>>(d, ar, it, p, 0);
-        else ks_up<FMT, 1, MINE><<<s.count, kSThreads, sm, stream>>>(d, ar, it, p, eval);
-    }
-    template <int FMT>
-    static void set_staged_smem(size_t mine, size_t opp) {
-        set_smem((const void*)ks_up<FMT, 0, true>, mine);
-        set_smem((const void*)ks_up<FMT, 1, true>, mine);
-        set_smem((const void*)ks_up<FMT, 0, false>, opp);
-        set_smem((const void*)ks_up<FMT, 1, false>, opp);
-    }
-    // Up sweep of one level's action nodes.  The staged engine launches the
-    // traverser's nodes and the opponent's separately (each launch's kernel is
-    // specialised for its side and sized for its shared memory).
+    // Up sweep of one level's action nodes.  The vector kernels take the
+    // traverser's nodes and the opponent's separately.
     // The action nodes of level l the level sweeps cover: all of them, or,
     // with river programs, those outside river betting rounds.
     Span act_level(int l, int actor) const {
         return use_river() ? plan.act_span_upper[actor][l] : plan.act_span_actor[actor][l];
     }
     void launch_up_level(int l, int p, int eval) {
-        if (staged) {
-            const Span mine = act_level(l, p), opp = act_level(l, 1 - p);
-            if (fmt == kFmtF32) {
-                staged_up<kDevF32, true>(mine, p, eval);
-                staged_up<kDevF32, false>(opp, p, eval);
-            } else if (fmt == kFmtFP8) {
-                staged_up<kDevFP8, true>(mine, p, eval);
-                staged_up<kDevFP8, false>(opp, p, eval);
-            } else {
-                staged_up<kDevI16, true>(mine, p, eval);
-                staged_up<kDevI16, false>(opp, p, eval);
-            }
+        if (vec) {
+            vec_up(d, ar, fmt, vnodes(act_level(l, p)), true, p, eval, stream);
+            vec_up(d, ar, fmt, vnodes(act_level(l, 1 - p)), false, p, eval, stream);
             return;
         }
         launch_up_action(plan.act_span[l], p, eval);
@@ -388,9 +368,9 @@ struct EngineImpl {
             else up_action<kDevI16, 8>(sa, p, eval);
         }
     }
-    void launch_down_action(const Span& sa, int mode) {
-        if (fmt == kFmtFP8) {  // the staged engine only
-            ks_down<kDevFP8><<<sa.count, kSThreads, st_down_smem, stream>>>(d, ar, snodes + sa.start, mode);
+    void launch_down_action(const Span& sa, int mode, int nh_launch) {
+        if (vec) {  // a launch that mixes actors is sized for the larger hand list
+            vec_down(d, ar, fmt, vnodes(sa), nh_launch, mode, stream);
             return;
         }
         if (fmt == kFmtF32) {
@@ -420,11 +400,12 @@ struct EngineImpl {
             if (use_river()) {  // two runs when both players' reach is refreshed
                 for (int q = 0; q < 2; q++) {
                     const Span sq = act_level(l, q);
-                    if ((qmask >> q & 1) && sq.count) timed(pr, 1, [&] { launch_down_action(sq, mode); });
+                    if ((qmask >> q & 1) && sq.count) timed(pr, 1, [&] { launch_down_action(sq, mode, d.nh[q]); });
                 }
             } else {
                 const Span sa = qmask == 3 ? plan.act_span[l] : plan.act_span_actor[qmask == 1 ? 0 : 1][l];
-                if (sa.count) timed(pr, 1, [&] { launch_down_action(sa, mode); });
+                const int nh = qmask == 3 ? std::max(d.nh[0], d.nh[1]) : d.nh[qmask == 1 ? 0 : 1];
+                if (sa.count) timed(pr, 1, [&] { launch_down_action(sa, mode, nh); });
             }
             const Span se = plan.edge_span[l];
             if (se.count)
@@ -719,6 +700,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     if (P.max_children > 32u) throw Error("an action node with more than 32 actions is not supported on the GPU");
     E.wide = P.max_children > 8u;
     E.staged = staged_kind && P.max_children <= (uint32_t)kSKA;
+    E.vec = staged_kind && P.max_children <= (uint32_t)kVKA;
     if (E.fmt == kFmtFP8 && !E.staged) throw Error("FP8 arenas need nodes of at most 4 actions (the staged kernels)");
     if (P.nh_max > kThreads * kMaxHpt) throw Error("more than 1536 hands per player is not supported on the GPU");
     CK(cudaStreamCreateWithFlags(&E.stream, cudaStreamNonBlocking));
@@ -788,77 +770,63 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     const size_t tsz = E.term64 ? sizeof(double) : sizeof(float);
     E.show_smem = (size_t)d.scr_elems * sizeof(double);
     if (E.warp) E.warp_smem = (size_t)kWarps * d.nh_pad * sizeof(float);
-    if (E.staged) {
-        // node records, packed hand words, fixed-stride card lists
-        PodVec<SNode> sn(P.act.size());
-        parallel_for((P.act.size() + 65535) / 65536, [&](size_t chunk) {
-          for (size_t k = chunk * 65536; k < std::min(P.act.size(), (chunk + 1) * 65536); k++) {
-            const ActItem& a = P.act[k];
-            SNode& x = sn[k];
-            std::memset(&x, 0, sizeof(x));
-            x.aoff = a.aoff;
-            x.cslot = a.cslot;
-            x.rslot = a.rslot;
-            x.oslot = a.oslot;
-            x.sidx = a.sidx;
-            x.actor = a.actor;
-            x.na = a.na;
-            x.fk = kNoSlot;
-            for (uint32_t c = 0; c < (uint32_t)kSKA; c++) {
-                x.cs[c] = kNoSlot;
-                x.rs[c] = kNoSlot;
-                if (c >= a.na) continue;
-                const ChildRef& r = P.crefs[a.cref + c];
-                x.cs[c] = r.cslot;
-                x.rs[c] = r.rslot;
-                if (r.kind == kChildFold) {
-                    const TermInfo& t = P.terms[r.term];
-                    x.fk = c;
-                    x.folder = t.aux;
-                    x.twin = t.twin;
-                    x.tlose = t.tlose;
+    if (E.vec) {
+        // node records, packed hand words
+        auto records = [&](auto KA) {
+            constexpr int K = KA();
+            PodVec<SNodeT<K>> sn(P.act.size());
+            parallel_for((P.act.size() + 65535) / 65536, [&](size_t chunk) {
+                for (size_t k = chunk * 65536; k < std::min(P.act.size(), (chunk + 1) * 65536); k++) {
+                    const ActItem& a = P.act[k];
+                    SNodeT<K>& x = sn[k];
+                    std::memset(&x, 0, sizeof(x));
+                    x.aoff = a.aoff;
+                    x.cslot = a.cslot;
+                    x.rslot = a.rslot;
+                    x.oslot = a.oslot;
+                    x.sidx = a.sidx;
+                    x.actor = a.actor;
+                    x.na = a.na;
+                    x.fk = kNoSlot;
+                    for (uint32_t c = 0; c < (uint32_t)K; c++) {
+                        x.cs[c] = kNoSlot;
+                        x.rs[c] = kNoSlot;
+                        if (c >= a.na) continue;
+                        const ChildRef& r = P.crefs[a.cref + c];
+                        x.cs[c] = r.cslot;
+                        x.rs[c] = r.rslot;
+                        if (r.kind == kChildFold) {
+                            const TermInfo& t = P.terms[r.term];
+                            x.fk = c;
+                            x.folder = t.aux;
+                            x.twin = t.twin;
+                            x.tlose = t.tlose;
+                        }
+                    }
                 }
-            }
-          }
-        });
-        E.snodes = dupload(sn, O, &B);
+            });
+            return dupload(sn, O, &B);
+        };
+        if (E.staged) E.snodes = records(std::integral_constant<int, kSKA>{});
+        else E.wnodes = records(std::integral_constant<int, kVKA>{});
         for (int q = 0; q < 2; q++) {
             const Hands& h = sp.hands[q];
-            std::vector<uint32_t> hi(h.c1.size());
-            for (size_t i = 0; i < hi.size(); i++) {
+            std::vector<uint32_t> hi((h.c1.size() + 3) / 4 * 4, 0u);  // whole groups of four
+            for (size_t i = 0; i < h.c1.size(); i++) {
                 const uint32_t s = sp.same[q][i];
                 hi[i] = (uint32_t)h.c1[i] | (uint32_t)h.c2[i] << 6 | (s == kSentinel ? 0xFFFFu : s) << 16;
             }
             d.hinfo[q] = dupload(hi, O, &B);
-            std::vector<uint16_t> h52(52 * 52, 0xFFFF);
-            for (int c = 0; c < 52; c++)
-                for (uint32_t k = P.hcard_off[q][c], j = 0; k < P.hcard_off[q][c + 1]; k++, j++) h52[c * 52 + j] = P.hcard_idx[q][k];
-            d.hcard52[q] = dupload(h52, O, &B);
         }
+    }
+    if (E.staged) {
         const int esz = fmt_bytes(E.fmt);
         E.st_mine_smem = SLayout(d.nh_pad, esz, E.pcfr, kSUpMine).total;
         E.st_opp_smem = SLayout(d.nh_pad, esz, E.pcfr, kSUpOpp).total;
         E.st_down_smem = SLayout(d.nh_pad, esz, E.pcfr, kSDown).total;
-        EngineImpl::set_staged_smem<kDevF32>(E.st_mine_smem, E.st_opp_smem);
-        EngineImpl::set_staged_smem<kDevI16>(E.st_mine_smem, E.st_opp_smem);
-        EngineImpl::set_staged_smem<kDevFP8>(E.st_mine_smem, E.st_opp_smem);
-        set_smem((const void*)ks_down<kDevF32>, E.st_down_smem);
-        set_smem((const void*)ks_down<kDevI16>, E.st_down_smem);
-        set_smem((const void*)ks_down<kDevFP8>, E.st_down_smem);
         E.show_pair_smem = show_pair_smem_bytes(d.nh_pad, (int)P.max_sorted);
         set_smem((const void*)ks_show_pair<128>, E.show_pair_smem);
         set_smem((const void*)ks_show_pair<256>, E.show_pair_smem);
-        const std::pair<const void*, int> show_fns[2] = {{(const void*)ks_show_pair<128>, 128},
-                                                         {(const void*)ks_show_pair<256>, 256}};
-        for (const auto& fn_nt : show_fns) {
-            cudaFuncAttributes fa;
-            CK(cudaFuncGetAttributes(&fa, fn_nt.first));
-            if ((size_t)fa.maxDynamicSharedSizeBytes < E.show_pair_smem || fa.maxThreadsPerBlock < fn_nt.second)
-                throw Error("showdown kernel limits: " + std::to_string(fa.maxDynamicSharedSizeBytes) +
-                            " B dynamic shared memory (needs " + std::to_string(E.show_pair_smem) + "), " +
-                            std::to_string(fa.maxThreadsPerBlock) + " threads, " + std::to_string(fa.numRegs) +
-                            " registers, " + std::to_string(fa.sharedSizeBytes) + " B static");
-        }
         setup_river(E, sp);
     }
     if (max_nterm && !E.warp) E.act_smem = (size_t)d.scr_elems * tsz + 2 * (size_t)max_nterm * d.nh_pad * sizeof(float);

@@ -1,0 +1,96 @@
+"""The default engine's node, showdown and chance kernels against the plain
+engine (one CTA and one launch per node kind, hands strided over the threads)
+on the same spots: the arithmetic is the same, so after a few iterations every
+arena entry, the exploitability and the root values are equal bit for bit.
+Sizes sit at the edges of the kernels' forms: the warp-per-node forms end at
+32, 64 and 128 hands, the showdown CTAs at 85, 170, 341 and 682 hands on a
+board, vectors come in groups of four."""
+import numpy as np
+import pytest
+
+import gtopen_b200 as g
+from gtopen_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _config(cards, n0, n1, bet, raise_, raises, seed, scale="%.6f", stack=400):
+    """n0 / n1 combos of a seeded board, weights in (0, 1]."""
+    rng = W.XorShift(seed)
+    board = W.draw_board(rng, cards)
+    combos = W.live_combos(board)
+    ranges = []
+    for n in (n0, n1):
+        order = sorted(range(len(combos)), key=lambda _: rng.next())[:n]
+        ranges.append(",".join("%s:%s" % (W.combo_str(*combos[i]), scale % (0.05 + 0.95 * rng.uniform()))
+                               for i in sorted(order)))
+    return {"board": "".join(W.card_str(c) for c in board), "range_oop": ranges[0], "range_ip": ranges[1],
+            "tree": W.tree_config(100, stack, bet, raise_, raises)}
+
+
+def _solve(cfg, engine, storage, fmt, algo, iters, lock):
+    spot = g.Spot(cfg)
+    host = g.Solver(spot, storage=storage, algo=algo)
+    if lock:
+        t = spot.tree()
+        for n in np.nonzero((t["kind"] == 0) & (t["nchild"] == 3))[0][:3]:
+            na, nh = int(t["nchild"][n]), spot.nh[int(t["player"][n])]
+            s = np.random.default_rng(int(n)).random((na, nh), np.float32)
+            host.set_lock(int(n), (s / s.sum(0)).reshape(-1))
+    gpu = g.GpuSolver(host, device_format=fmt, engine=engine)
+    gpu.iterate(iters)
+    out = [gpu.exploitability()]
+    out += [gpu.root_cfv(p, mode) for p in (0, 1) for mode in (0, 1)]
+    gpu.iterate(1)  # after the evaluation sweeps rewrote the reach slots
+    which = (0, 1, 2) if algo == "pcfr+" else (0, 1)
+    return out + [gpu.export_arena(w, p) for w in which for p in (0, 1)]
+
+
+def _equal(cfg, storage="f32", fmt=None, algo="dcfr", iters=3, lock=False):
+    a = _solve(cfg, "staged", storage, fmt, algo, iters, lock)
+    b = _solve(cfg, "plain", storage, fmt, algo, iters, lock)
+    assert a[0] == b[0]
+    for x, y in zip(a[1:], b[1:]):
+        np.testing.assert_array_equal(x, y)
+    assert all(np.isfinite(x).all() for x in a[1:])
+
+
+FORMATS = [("f32", None, "dcfr"), ("compressed", None, "dcfr"), ("compressed", "i16sr", "dcfr"),
+           ("f32", None, "pcfr+"), ("compressed", None, "pcfr+"), ("compressed", None, "cfr+")]
+
+
+@pytest.mark.parametrize("storage,fmt,algo", FORMATS)
+@pytest.mark.parametrize("n0,n1", [(1, 2), (31, 33), (32, 64), (65, 63), (127, 129), (128, 341), (130, 1081)])
+def test_river_sizes(n0, n1, storage, fmt, algo):
+    _equal(_config(5, n0, n1, ("33", "75", "a"), ("2.5x",), 1, seed=100 + n0), storage, fmt, algo)
+
+
+@pytest.mark.parametrize("storage,fmt,algo", FORMATS)
+@pytest.mark.parametrize("n0,n1", [(3, 5), (30, 90), (200, 171), (600, 100)])
+def test_turn_sizes(n0, n1, storage, fmt, algo):
+    _equal(_config(4, n0, n1, ("75",), ("2.5x",), 1, seed=n0), storage, fmt, algo)
+
+
+@pytest.mark.parametrize("bets", [4, 6, 7])
+@pytest.mark.parametrize("storage,fmt,algo", FORMATS)
+def test_wide_nodes(bets, storage, fmt, algo):
+    """5 to 8 actions at a node (check and 4 to 7 sizes): the wide records."""
+    sizes = ("10", "20", "30", "45", "60", "80", "100")[:bets]
+    _equal(_config(5, 150, 37, sizes, ("2.5x",), 1, seed=bets, stack=1000), storage, fmt, algo)
+
+
+@pytest.mark.parametrize("storage,fmt,algo", FORMATS)
+def test_locked_nodes(storage, fmt, algo):
+    _equal(_config(4, 61, 142, ("33", "75"), ("2.5x",), 1, seed=9), storage, fmt, algo, lock=True)
+
+
+@pytest.mark.parametrize("scale", ["%.6fe-20", "%.6fe-32", "%.6fe-37"])
+def test_tiny_weights(scale):
+    """Weights whose fixed-point scales pass 2^100 and 2^126."""
+    _equal(_config(5, 90, 70, ("75",), ("2.5x",), 1, seed=4, scale=scale))
+
+
+def test_suit_symmetric_flop():
+    cfg = W.iso_spot()
+    _equal(cfg)
+    _equal(cfg, "compressed", "i16sr")
