@@ -1,0 +1,387 @@
+// Showdown kernel of the level sweeps (the default engine).
+//
+// kv_show: one CTA evaluates G showdowns of one river board at once
+// (game.rs:501-577 with the plan's rank tables), all of a sweep's showdowns
+// in one launch -- they read only reach vectors, so no level waits for
+// another.  Exact sums (cfr_dev.cuh), so the split changes no bits.
+//
+// What bounds it and why this layout: a hand's value needs eight prefix sums
+// at positions of its own (strength order below / not above it, its two
+// cards' lists likewise, the two cards' totals), i.e. eight scattered
+// shared-memory reads, and shared-memory wavefronts and the instructions
+// around them set the time (470 v 647 hands: LSU wavefronts 67% and issue 52%
+// of their peaks, DRAM 9%).
+//   * The G showdowns of a board use the same positions, so the prefixes lie
+//     row by row with the G sums side by side and a lane takes two showdowns
+//     (one 16-byte access): at G = 8 a quarter warp reads whole rows.
+//   * The segmented scan over [strength order | card lists] keeps a lane's K
+//     entries in registers (K up to 16) until its carry is known, so every
+//     row is written once.
+//   * The fewest threads whose lanes hold the scan, then the largest G: the
+//     per-warp work (shuffles, carries, address set-up) is paid by fewer
+//     warps.  Measured, ms per iteration for both sweeps (threads x G):
+//     28 v 23 hands 64x8 0.077, 128x8 0.111, 64x2 0.199; 64 v 39 hands 64x8
+//     0.246, 128x8 0.288, 64x2 0.443; 243 v 321 64x2 2.35, 128x4 2.43, 256x8
+//     2.70; 470 v 647 128x2 1.45, 256x4 1.65, 512x8 2.12.
+// Showdowns of one iteration before (two at a time, one launch per level,
+// chunks rewritten after the scan) -> after: 28 v 23 hands 0.41 -> 0.08 ms,
+// 64 v 39 0.87 -> 0.25, 243 v 321 3.21 -> 2.35, 470 v 647 2.25 -> 1.45, a turn
+// of 3,696 showdowns 0.43 -> 0.066, a river 0.14 -> 0.026.
+#include "cfr_vec.hpp"
+
+#include <type_traits>
+
+namespace gtob {
+namespace {
+
+template <class T>
+__device__ __forceinline__ T pick(T const (&x)[2], int a) { return a ? x[1] : x[0]; }
+
+// A board's scan entries: the opponent's hands in strength order (m), then
+// card by card each list of the hands holding the card, in strength order
+// (2 m); bit 15 marks the first entry of the strength order and of each list.
+// Lanes scan K consecutive entries each; entry f's running sum goes to row
+// f + 1 + f / K (a row left free per K entries spreads the lanes' stores over
+// the banks), row 0 is zero: the empty prefix of every list.
+__host__ __device__ inline int show_entries(int m, int K) { return (3 * m + K - 1) / K * K; }
+__host__ __device__ inline int show_rows(int m, int K) { return show_entries(m, K) / K * (K + 1) + 1; }
+__host__ __device__ inline int show_img_len(int msort, int K) { return (show_entries(msort, K) + 7) & ~7; }
+__device__ __forceinline__ int show_row(int entries, int K) {  // the row of the sum of a list's entries up to `entries`
+    return entries + (entries - 1) / K;
+}
+struct ShowLayout {
+    unsigned o_r, o_img, total;
+    __host__ __device__ ShowLayout(int G, int K, int msort, int nho_pad) {
+        o_r = (unsigned)show_rows(msort, K) * (unsigned)G * 8u;
+        o_img = o_r + (unsigned)nho_pad * (unsigned)G * 4u;  // nho_pad is a multiple of 4
+        total = o_img + (unsigned)show_img_len(msort, K) * 2u;
+    }
+};
+
+// Per board and traverser hand: the rows of its eight sums (strictly weaker
+// and not stronger hands; the same for each of its cards' lists; the lists'
+// totals); s1 of a blocked hand: 0xFFFF.
+struct alignas(16) HandRank {
+    uint16_t lb, ub, q1lo, q1hi, q2lo, q2hi, s1, s2;
+};
+
+// A vector's scaling onto its grid and back (fix_q, fix_f).  Up to S = 126
+// one multiplication does what their two-step form does: the power of two is
+// a normal number, the way to the grid is exact, and the way back rounds
+// once.  BIG: some lane's vector is smaller than that.
+struct Grid {
+    int S;
+    float up, down;
+};
+__device__ __forceinline__ Grid make_grid(float mx) {
+    Grid g;
+    g.S = fix_scale(mx);
+    g.up = pow2f(min(g.S, 126));
+    g.down = pow2f(-min(g.S, 126));
+    return g;
+}
+template <bool BIG>
+__device__ __forceinline__ long long grid_q(const Grid& g, float r) {
+    return BIG ? fix_q(r, g.S) : __float2ll_rn(__fmul_rn(r, g.up));
+}
+template <bool BIG>
+__device__ __forceinline__ float grid_f(const Grid& g, long long v) {
+    return BIG ? fix_f(v, g.S) : __fmul_rn(__ll2float_rn(v), g.down);
+}
+struct ShowPay {
+    float win, lose, tie;
+};
+// One hand's value from its integer sums (game.rs:560-575).
+template <bool BIG>
+__device__ __forceinline__ float show_value(const Grid& g, const ShowPay& pay, long long low, long long notabove,
+                                            long long all, float same) {
+    const float lower = grid_f<BIG>(g, low);
+    const float higher = grid_f<BIG>(g, all - notabove);
+    const float valid = grid_f<BIG>(g, all) + same;
+    const float tied = valid - lower - higher;
+    return pay.win * lower + pay.lose * higher + pay.tie * tied;
+}
+__device__ __forceinline__ longlong2 shfl_up2(const longlong2& v, int x) {
+    return make_longlong2(__shfl_up_sync(0xffffffffu, v.x, x), __shfl_up_sync(0xffffffffu, v.y, x));
+}
+
+template <int G, int NT, int K, bool BIG>
+__device__ __forceinline__ void show_group(const Dev& d, unsigned char* sm, const ShowLayout& SL, const ShowItem* s_it,
+                                           longlong2* s_w, int* s_wf, const Grid& ga, const Grid& gb, int m, int nhp,
+                                           const HandRank* hr, const uint32_t* hinfo) {
+    constexpr int L = G / 2, NC = NT / L, NW = NT / 32;
+    const int tid = (int)threadIdx.x, l = tid & (L - 1), c_ = tid / L, lane = tid & 31, warp = tid >> 5;
+    longlong2* U = (longlong2*)sm + l;  // row k: U[k * L]
+    const float2* r2 = (const float2*)(sm + SL.o_r) + l;
+    // the lane's K entries: running sums since the last list head
+    const bool on = c_ * K < 3 * m;
+    longlong2 a = make_longlong2(0, 0), loc[K];
+    int first = K;  // the first head among them
+    if (on) {
+        const uint2* ent = (const uint2*)(sm + SL.o_img) + c_ * (K / 4);
+#pragma unroll
+        for (int k = 0; k < K; k += 4) {
+            const uint2 w = ent[k / 4];
+            const uint32_t e[4] = {w.x & 0xFFFFu, w.x >> 16, w.y & 0xFFFFu, w.y >> 16};
+            float2 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] = r2[(e[j] & 0x7FFFu) * L];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (e[j] & 0x8000u) {
+                    a = make_longlong2(0, 0);
+                    first = min(first, k + j);
+                }
+                a.x += grid_q<BIG>(ga, x[j].x);
+                a.y += grid_q<BIG>(gb, x[j].y);
+                loc[k + j] = a;
+            }
+        }
+    }
+    // scan of the lanes' (head seen, sum) pairs over the lanes with this l
+    bool fl = first < K;
+#pragma unroll
+    for (int x = L; x < 32; x <<= 1) {
+        const int fu = __shfl_up_sync(0xffffffffu, (int)fl, x);
+        const longlong2 u = shfl_up2(a, x);
+        if (lane >= x) {
+            if (!fl) {
+                a.x += u.x;
+                a.y += u.y;
+            }
+            fl = fl || fu;
+        }
+    }
+    longlong2 c = shfl_up2(a, L);  // what the warp's lanes before this one carry over
+    bool cf = __shfl_up_sync(0xffffffffu, (int)fl, L) != 0;
+    if (lane < L) {
+        c = make_longlong2(0, 0);
+        cf = false;
+    }
+    if (lane >= 32 - L) {
+        s_w[warp * L + l] = a;
+        if (l == 0) s_wf[warp] = (int)fl;
+    }
+    __syncthreads();
+    if (!cf) {  // and the warps before it, back to the last head
+#pragma unroll
+        for (int w = NW - 2; w >= 0; w--) {
+            if (w < warp && !cf) {
+                const longlong2 u = s_w[w * L + l];
+                c.x += u.x;
+                c.y += u.y;
+                cf = s_wf[w] != 0;
+            }
+        }
+    }
+    if (tid < L) *U = make_longlong2(0, 0);
+    if (on) {
+        longlong2* dst = U + (c_ * (K + 1) + 1) * L;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            longlong2 v = loc[k];
+            if (k < first) {
+                v.x += c.x;
+                v.y += c.y;
+            }
+            dst[k * L] = v;
+        }
+    }
+    __syncthreads();
+    // values, in hand order: a warp's rows of output are whole sectors
+    const ShowItem &ia = s_it[2 * l], &ib = s_it[2 * l + 1];
+    float* outA = d.cfv + (size_t)ia.cslot * d.nh_max;
+    float* outB = d.cfv + (size_t)ib.cslot * d.nh_max;
+    const bool onA = ia.cslot != kNoSlot, onB = ib.cslot != kNoSlot;
+    const ShowPay pa{ia.twin, ia.tlose, ia.ttie}, pb{ib.twin, ib.tlose, ib.ttie};
+    const longlong2 T = U[m > 0 ? show_row(m, K) * L : 0];
+    HandRank next;
+    uint32_t nexth = 0;
+    if (c_ < nhp) {
+        next = hr[c_];
+        nexth = hinfo[c_];
+    }
+    for (int i = c_; i < nhp; i += NC) {
+        const HandRank e = next;
+        const uint32_t same = nexth >> 16;
+        if (i + NC < nhp) {  // in flight during this hand's sums
+            next = hr[i + NC];
+            nexth = hinfo[i + NC];
+        }
+        float vA = 0.0f, vB = 0.0f;  // a blocked hand's value
+        if (e.s1 != 0xFFFFu) {
+            const longlong2 plb = U[(int)e.lb * L], pub = U[(int)e.ub * L], q1l = U[(int)e.q1lo * L],
+                            q1h = U[(int)e.q1hi * L], q2l = U[(int)e.q2lo * L], q2h = U[(int)e.q2hi * L],
+                            s1 = U[(int)e.s1 * L], s2 = U[(int)e.s2 * L];
+            float2 sr = make_float2(0.0f, 0.0f);
+            if (same != 0xFFFFu) sr = r2[(int)same * L];
+            vA = show_value<BIG>(ga, pa, plb.x - q1l.x - q2l.x, pub.x - q1h.x - q2h.x, T.x - s1.x - s2.x, sr.x);
+            vB = show_value<BIG>(gb, pb, plb.y - q1l.y - q2l.y, pub.y - q1h.y - q2h.y, T.y - s1.y - s2.y, sr.y);
+        }
+        if (onA) outA[i] = vA;
+        if (onB) outB[i] = vB;
+    }
+}
+
+template <int G, int NT, int K>
+__global__ void __launch_bounds__(NT) kv_show(Dev d, const ShowItem* items, const uint16_t* img, const HandRank* ranks,
+                                              int p, int msort) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ longlong2 s_w[NT / 32 * (G / 2)];
+    __shared__ int s_wf[NT / 32];
+    __shared__ uint32_t s_mx[G];
+    __shared__ ShowItem s_it[G];
+    const int o = 1 - p, nho = pick(d.nh, o), nhp = pick(d.nh, p);
+    const int nho_pad = (nho + 3) & ~3;
+    const ShowLayout SL(G, K, msort, nho_pad);
+    const int tid = (int)threadIdx.x, il = show_img_len(msort, K);
+    const int g = tid & (G - 1);
+    const ShowItem it = items[(size_t)blockIdx.x * G + g];  // (every thread: its own vector's; the slot is the batch's)
+    if (tid < G) {
+        s_mx[tid] = 0u;
+        s_it[tid] = it;
+    }
+    const uint32_t slot = it.slot;
+    const int m = (int)pick(d.sorted_cnt, o)[slot];
+    {  // the board's entries
+        const uint4* src = (const uint4*)(img + (size_t)slot * il);
+        uint4* im = (uint4*)(sm + SL.o_img);
+        for (int k = tid; k < il / 8; k += NT) im[k] = src[k];
+    }
+    uint32_t mx = 0u;
+    {  // the reach vectors, interleaved by showdown: four hands a load
+        const int q4 = nho_pad >> 2;
+        const bool live = it.cslot != kNoSlot;
+        const float* src = pick(d.reach, o) + (size_t)it.rs[o] * pick(d.rstr, o);
+        float* r = (float*)(sm + SL.o_r);
+        for (int q = tid / G; q < q4; q += NT / G) {
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (live) v = ((const float4*)src)[q];
+            const float x[4] = {v.x, 4 * q + 1 < nho ? v.y : 0.0f, 4 * q + 2 < nho ? v.z : 0.0f,
+                                4 * q + 3 < nho ? v.w : 0.0f};
+            mx = max(mx, __float_as_uint(fmaxf(fmaxf(fmaxf(x[0], 0.0f), x[1]), fmaxf(fmaxf(x[2], 0.0f), x[3]))));
+#pragma unroll
+            for (int j = 0; j < 4; j++) {  // rotated so that the warp's quads write different banks
+                const int k = (j + q) & 3;
+                const float y = k == 0 ? x[0] : k == 1 ? x[1] : k == 2 ? x[2] : x[3];
+                r[(4 * q + k) * G + g] = y;
+            }
+        }
+    }
+#pragma unroll
+    for (int x = G; x < 32; x <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+    __syncthreads();
+    if ((tid & 31) < G) atomicMax(&s_mx[g], mx);
+    __syncthreads();
+    const int l = tid & (G / 2 - 1);
+    const Grid ga = make_grid(__uint_as_float(s_mx[2 * l])), gb = make_grid(__uint_as_float(s_mx[2 * l + 1]));
+    const HandRank* hr = ranks + (size_t)slot * nhp;
+    // every warp holds every lane number l, so all warps agree
+    if (__any_sync(0xffffffffu, ga.S > 126 || gb.S > 126))
+        show_group<G, NT, K, true>(d, sm, SL, s_it, s_w, s_wf, ga, gb, m, nhp, hr, pick(d.hinfo, p));
+    else
+        show_group<G, NT, K, false>(d, sm, SL, s_it, s_w, s_wf, ga, gb, m, nhp, hr, pick(d.hinfo, p));
+}
+
+// The boards' rank entries by hand, for kv_show (once per engine).
+__global__ void k_hand_ranks(Dev d, int p, int K, HandRank* out) {
+    const uint32_t slot = blockIdx.x;
+    const int nh = pick(d.nh, p), o = 1 - p;
+    HandRank* row = out + (size_t)slot * nh;
+    for (int i = threadIdx.x; i < nh; i += blockDim.x) row[i] = HandRank{0, 0, 0, 0, 0, 0, 0xFFFF, 0};
+    __syncthreads();
+    const RankEntry* in = pick(d.rank, p) + pick(d.rank_off, p)[slot];
+    const uint32_t cnt = pick(d.rank_cnt, p)[slot];
+    const uint32_t* coff = pick(d.ccard_off, o) + (size_t)slot * 53;
+    const int m = (int)pick(d.sorted_cnt, o)[slot];
+    for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x) {
+        const RankEntry e = in[k];
+        const int c1 = e.cards & 0xFF, c2 = e.cards >> 8;
+        auto strength = [&](int n) { return (uint16_t)(n ? show_row(n, K) : 0); };
+        // the plan counts a card's prefixes from its offset + card number
+        auto list = [&](int c, int n) { return (uint16_t)(n ? show_row(m + (int)(coff[c] - coff[0]) + n, K) : 0); };
+        auto prefix = [&](int c, int q) { return list(c, q - (int)(coff[c] - coff[0]) - c); };
+        auto total = [&](int c) { return list(c, (int)(coff[c + 1] - coff[c])); };
+        row[e.idx] = HandRank{strength(e.lb),    strength(e.ub),    prefix(c1, e.q1lo), prefix(c1, e.q1hi),
+                              prefix(c2, e.q2lo), prefix(c2, e.q2hi), total(c1),          total(c2)};
+    }
+}
+// Every board's scan entries of player o's hands.
+__global__ void k_show_images(Dev d, int o, int msort, int K, uint16_t* out) {
+    const uint32_t slot = blockIdx.x;
+    const int il = show_img_len(msort, K), m = (int)pick(d.sorted_cnt, o)[slot];
+    uint16_t* im = out + (size_t)slot * il;
+    const uint32_t* coff = pick(d.ccard_off, o) + (size_t)slot * 53;
+    const uint16_t* order = pick(d.sorted_idx, o) + pick(d.sorted_off, o)[slot];
+    const uint8_t* card = pick(d.ccard_card, o) + coff[0];
+    const uint16_t* pos = pick(d.ccard_pos, o) + coff[0];
+    for (int f = threadIdx.x; f < il; f += blockDim.x) {
+        uint16_t e = 0;  // beyond the last list: read, never used
+        if (f < m) {
+            e = (uint16_t)(order[f] | (f == 0 ? 0x8000u : 0u));
+        } else if (f < 3 * m) {
+            const int t = f - m;
+            e = (uint16_t)(order[pos[t]] | (t == 0 || card[t - 1] != card[t] ? 0x8000u : 0u));
+        }
+        im[f] = e;
+    }
+}
+
+template <class F>
+bool with_show(const ShowShape& sh, F f) {
+    auto by_k = [&](auto G, auto NT) {
+        if (sh.chunk == 4) f(G, NT, std::integral_constant<int, 4>{});
+        else if (sh.chunk == 8) f(G, NT, std::integral_constant<int, 8>{});
+        else if (sh.chunk == 12) f(G, NT, std::integral_constant<int, 12>{});
+        else if (sh.chunk == 16) f(G, NT, std::integral_constant<int, 16>{});
+        else return false;
+        return true;
+    };
+    using C8 = std::integral_constant<int, 8>;
+    using C4 = std::integral_constant<int, 4>;
+    using C2 = std::integral_constant<int, 2>;
+    if (sh.threads == 64 && sh.group == 8) return by_k(C8{}, std::integral_constant<int, 64>{});
+    if (sh.threads == 64 && sh.group == 4) return by_k(C4{}, std::integral_constant<int, 64>{});
+    if (sh.threads == 64 && sh.group == 2) return by_k(C2{}, std::integral_constant<int, 64>{});
+    if (sh.threads == 128 && sh.group == 2) return by_k(C2{}, std::integral_constant<int, 128>{});
+    if (sh.threads == 256 && sh.group == 2) return by_k(C2{}, std::integral_constant<int, 256>{});
+    return false;
+}
+}  // namespace
+
+bool show_shape(int group, int max_sorted, ShowShape& sh) {
+    for (int threads = 64; threads <= (group == 2 ? 256 : 64); threads *= 2) {
+        const int rows = threads / (group / 2), k = (3 * max_sorted + rows - 1) / rows;
+        sh = {group, threads, k <= 4 ? 4 : (k + 3) / 4 * 4};
+        if (sh.chunk <= 16) return true;
+    }
+    return false;
+}
+size_t show_group_smem(const ShowShape& sh, int max_sorted, int nho) {
+    return ShowLayout(sh.group, sh.chunk, max_sorted, (nho + 3) & ~3).total;
+}
+const void* show_group_kernel(const ShowShape& sh) {
+    const void* fn = nullptr;
+    with_show(sh, [&](auto G, auto NT, auto K) { fn = (const void*)kv_show<G(), NT(), K()>; });
+    return fn;
+}
+size_t hand_rank_bytes() { return sizeof(HandRank); }
+size_t show_image_bytes(const ShowShape& sh, int max_sorted) { return (size_t)show_img_len(max_sorted, sh.chunk) * 2; }
+void build_show_tables(const Dev& d, const ShowGroups& sg, uint32_t slots, cudaStream_t s) {
+    if (!slots) return;
+    for (int q = 0; q < 2; q++) {  // ranks of traverser q among the other player's entries
+        k_hand_ranks<<<slots, 256, 0, s>>>(d, q, sg.shape[1 - q].chunk, (HandRank*)sg.ranks[q]);
+        k_show_images<<<slots, 256, 0, s>>>(d, q, sg.max_sorted[q], sg.shape[q].chunk, (uint16_t*)sg.img[q]);
+    }
+}
+void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s) {
+    if (!sg.count) return;
+    const int o = 1 - p;
+    const size_t smem = show_group_smem(sg.shape[o], sg.max_sorted[o], d.nh[o]);
+    with_show(sg.shape[o], [&](auto G, auto NT, auto K) {
+        kv_show<G(), NT(), K()><<<sg.count, NT(), smem, s>>>(d, sg.items, (const uint16_t*)sg.img[o],
+                                                             (const HandRank*)sg.ranks[p], p, sg.max_sorted[o]);
+    });
+}
+
+}  // namespace gtob

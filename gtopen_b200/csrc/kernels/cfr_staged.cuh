@@ -1029,12 +1029,5 @@ __device__ bool show_batch_run(const Dev& d, const ShowItem* items, const ShowBa
     }
     return true;
 }
-template <int NT>
-__global__ void __launch_bounds__(NT) ks_show_pair(Dev d, const ShowItem* items, const ShowBatch* batches, int p,
-                                                    int msort) {
-    extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ ShowShared<NT> ss;
-    show_batch_run<NT>(d, items, batches[blockIdx.x], p, msort, sm, ss);
-}
 
 }  // namespace gtob

@@ -21,5 +21,29 @@ void vec_down(const Dev& d, const Arenas& ar, int fmt, const VecNodes& n, int nh
 // eval < 0: the CFR update; 0 / 1: best response / average-strategy values.
 void vec_up(const Dev& d, const Arenas& ar, int fmt, const VecNodes& n, bool mine, int p, int eval, cudaStream_t s);
 
+// A sweep's showdowns in batches of `group` of one river board, one CTA each;
+// a short batch is filled with items without a cfv slot.
+struct ShowShape {
+    int group = 8;      // showdowns per batch: 2, 4 or 8
+    int threads = 64;   // per CTA
+    int chunk = 4;      // scan entries per lane: 4, 8, 12 or 16
+};
+struct ShowGroups {
+    const ShowItem* items = nullptr;  // count * group
+    uint32_t count = 0;
+    ShowShape shape[2];                   // per player whose hands are scanned (one group for both)
+    int max_sorted[2] = {0, 0};           // per player: most hands on a board
+    void* ranks[2] = {nullptr, nullptr};  // per traverser: every board's rank entries by hand
+    void* img[2] = {nullptr, nullptr};    // per player: every board's scan entries
+};
+// The CTA for boards of at most max_sorted opponent hands: the fewest threads
+// whose lanes hold the scan; false if none.
+bool show_shape(int group, int max_sorted, ShowShape& sh);
+size_t show_group_smem(const ShowShape& sh, int max_sorted, int nho);
+const void* show_group_kernel(const ShowShape& sh);
+size_t hand_rank_bytes();
+size_t show_image_bytes(const ShowShape& sh, int max_sorted);
+void build_show_tables(const Dev& d, const ShowGroups& sg, uint32_t slots, cudaStream_t s);
+void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s);
 
 }  // namespace gtob

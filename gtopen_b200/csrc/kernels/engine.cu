@@ -117,6 +117,7 @@ struct EngineImpl {
     FoldItem* fold = nullptr;
     ShowItem* show = nullptr;
     ShowBatch* show_batch = nullptr;
+    ShowGroups shows, shows_upper;  // vector kernels: every showdown / those outside river rounds
     ChanceItem* chance = nullptr;
     XNode* xnodes[2] = {nullptr, nullptr};
     std::vector<XNode> hx[2];
@@ -440,7 +441,13 @@ struct EngineImpl {
         // stream, every level of them, beside the chain of chance and action
         // levels; the chain waits for level l + 1's terminals before it
         // consumes them at level l.
-        const bool fork = pr == nullptr && side != nullptr;
+        // The vector kernels' showdowns are one launch for all levels, on the
+        // chain itself: it fills the device, and every level below needs some.
+        const bool fork = pr == nullptr && side != nullptr && !vec;
+        if (vec) {
+            const ShowGroups& sg = use_river() ? shows_upper : shows;
+            if (sg.count) timed(pr, 4, [&] { vec_show(d, sg, p, stream); });
+        }
         if (fork) {
             CK(cudaEventRecord(ev_fork, stream));
             CK(cudaStreamWaitEvent(side, ev_fork, 0));
@@ -450,7 +457,8 @@ struct EngineImpl {
             }
         }
         for (int l = L - 1; l >= 0; l--) {
-            if (!fork) launch_terminals(l, p, stream, pr);
+            if (vec) {
+            } else if (!fork) launch_terminals(l, p, stream, pr);
             else if (l + 1 < L) CK(cudaStreamWaitEvent(stream, ev_term[l + 1], 0));
             reduce_level(l, p);  // a shard: the children of this level's top chance nodes from every shard
             const Span sc = plan.chance_span[l];
@@ -484,20 +492,7 @@ struct EngineImpl {
         const Span sf = plan.fold_span[l];
         if (sf.count) timed(pr, 3, [&] { k_fold<<<sf.count, kThreads, 0, st>>>(d, fold + sf.start, p); });
         const Span ss = plan.show_span[l];
-        const Span sb = use_river() ? plan.show_batch_span_upper[l] : plan.show_batch_span[l];
-        if (staged ? sb.count > 0 : ss.count > 0)
-            timed(pr, 4, [&] {
-                if (staged) {
-                    if (plan.max_sorted > 384)
-                        ks_show_pair<256><<<sb.count, 256, show_pair_smem, st>>>(d, show, show_batch + sb.start, p,
-                                                                                  (int)plan.max_sorted);
-                    else
-                        ks_show_pair<128><<<sb.count, 128, show_pair_smem, st>>>(d, show, show_batch + sb.start, p,
-                                                                                  (int)plan.max_sorted);
-                } else {
-                    k_showdown<<<ss.count, kThreads, show_smem, st>>>(d, show + ss.start, p);
-                }
-            });
+        if (ss.count) timed(pr, 4, [&] { k_showdown<<<ss.count, kThreads, show_smem, st>>>(d, show + ss.start, p); });
     }
     void record_iteration() {
         k_begin_iteration<<<1, 1, 0, stream>>>(d.iter, d.disc, algo);
@@ -663,6 +658,75 @@ static void setup_river(EngineImpl& E, const Spot& sp) {
     E.river = true;
 }
 
+// The vector kernels' showdown batches over all levels, sorted by river board,
+// and the boards' tables.  G showdowns share a CTA: 8 where that leaves a CTA
+// for every SM and its prefixes fit, else 4 or 2 (a river spot has one board
+// and a dozen showdowns: narrow batches keep more SMs busy).
+static void setup_shows(EngineImpl& E) {
+    const Plan& P = E.plan;
+    Dev& d = E.d;
+    if (P.show.empty()) return;
+    int dev = 0, optin = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    std::vector<uint32_t> per(P.num_slots, 0);
+    for (const ShowItem& x : P.show) per[x.slot]++;
+    ShowGroups sg;
+    for (int q = 0; q < 2; q++)
+        for (uint32_t c : P.sorted_cnt[q]) sg.max_sorted[q] = std::max(sg.max_sorted[q], (int)c);
+    for (int group = 8; group >= 2; group /= 2) {
+        uint64_t batches = 0;
+        for (uint32_t c : per) batches += (c + group - 1) / group;
+        if (batches < (uint64_t)nsm && group > 2) continue;
+        bool fits = true;
+        for (int q = 0; q < 2; q++)
+            fits = fits && show_shape(group, sg.max_sorted[q], sg.shape[q]) &&
+                   show_group_smem(sg.shape[q], sg.max_sorted[q], P.nh[q]) + 2048 <= (size_t)optin;
+        if (fits) break;
+        if (group == 2) throw Error("showdown kernel: more hands on a board than it takes");
+    }
+    auto& O = E.owned;
+    size_t& B = E.bytes;
+    for (int q = 0; q < 2; q++) {
+        sg.ranks[q] = dalloc((size_t)P.num_slots * P.nh[q] * hand_rank_bytes(), O, &B);
+        sg.img[q] = dalloc((size_t)P.num_slots * show_image_bytes(sg.shape[q], sg.max_sorted[q]), O, &B);
+    }
+    CK(cudaStreamSynchronize(0));  // the tables' zeroing, before the engine's own (non-blocking) stream writes them
+    build_show_tables(d, sg, P.num_slots, E.stream);
+    CK(cudaGetLastError());
+    auto group = [&](bool upper_only) {
+        ShowGroups g = sg;
+        std::vector<uint32_t> at(P.num_slots + 1, 0);
+        auto each = [&](auto f) {
+            for (size_t l = 0; l < P.show_batch_span.size(); l++) {
+                const Span s = upper_only ? P.show_batch_span_upper[l] : P.show_batch_span[l];
+                for (uint32_t b = s.start; b < s.start + s.count; b++)
+                    for (uint32_t k = 0; k < P.show_batch[b].count; k++) f(P.show[P.show_batch[b].start + k]);
+            }
+        };
+        each([&](const ShowItem& x) { at[x.slot + 1]++; });
+        const uint32_t G = (uint32_t)g.shape[0].group;
+        std::vector<uint32_t> slot_of;  // per batch
+        for (uint32_t s = 0; s < P.num_slots; s++) {
+            const uint32_t nb = (at[s + 1] + G - 1) / G;
+            slot_of.insert(slot_of.end(), nb, s);
+            at[s + 1] = at[s] + nb * G;
+        }
+        PodVec<ShowItem> it(slot_of.size() * G);
+        for (size_t b = 0; b < slot_of.size(); b++)
+            for (uint32_t k = 0; k < G; k++) it[b * G + k] = ShowItem{kNoSlot, {0, 0}, slot_of[b], 0.0f, 0.0f, 0.0f, 0};
+        each([&](const ShowItem& x) { it[at[x.slot]++] = x; });
+        g.items = dupload(it, O, &B);
+        g.count = (uint32_t)slot_of.size();
+        return g;
+    };
+    E.shows = group(false);
+    if (E.river) E.shows_upper = group(true);
+    for (int q = 0; q < 2; q++)
+        set_smem(show_group_kernel(sg.shape[q]), show_group_smem(sg.shape[q], sg.max_sorted[q], P.nh[q]));
+}
+
 // --------------------------------------------------------------- GpuEngine
 GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine) : GpuEngine(host, fmt, engine, 0, 1, nullptr) {}
 
@@ -825,10 +889,9 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
         E.st_opp_smem = SLayout(d.nh_pad, esz, E.pcfr, kSUpOpp).total;
         E.st_down_smem = SLayout(d.nh_pad, esz, E.pcfr, kSDown).total;
         E.show_pair_smem = show_pair_smem_bytes(d.nh_pad, (int)P.max_sorted);
-        set_smem((const void*)ks_show_pair<128>, E.show_pair_smem);
-        set_smem((const void*)ks_show_pair<256>, E.show_pair_smem);
         setup_river(E, sp);
     }
+    if (E.vec) setup_shows(E);
     if (max_nterm && !E.warp) E.act_smem = (size_t)d.scr_elems * tsz + 2 * (size_t)max_nterm * d.nh_pad * sizeof(float);
     if (runouts) E.chance_smem = (size_t)d.scr_elems * tsz + 2 * (size_t)d.nh_pad * sizeof(float);
     set_smem((const void*)k_showdown, E.show_smem);
