@@ -1,4 +1,4 @@
-// Showdown kernel of the level sweeps (the default engine).
+// Showdown and chance kernels of the level sweeps (the default engine).
 //
 // kv_show: one CTA evaluates G showdowns of one river board at once
 // (game.rs:501-577 with the plan's rank tables), all of a sweep's showdowns
@@ -27,6 +27,15 @@
 // chunks rewritten after the scan) -> after: 28 v 23 hands 0.41 -> 0.08 ms,
 // 64 v 39 0.87 -> 0.25, 243 v 321 3.21 -> 2.35, 470 v 647 2.25 -> 1.45, a turn
 // of 3,696 showdowns 0.43 -> 0.066, a river 0.14 -> 0.026.
+//
+// kv_chance, kv_edges: a chance node's value and its edges' reach, one hand
+// (four, for the edges) per thread, so that a level of a few nodes still
+// spreads over the chip: a node's 48 children used to be read one after the
+// other by one CTA per node, 60-85 us a level however few its nodes.  Both
+// are bound by the latency of their loads on small levels and by HBM on
+// large ones.  One iteration, before -> after: chance values of a 564-hand
+// turn 0.47 -> 0.09 ms, of a 470 v 647 flop 1.00 -> 0.26; the flop's edges
+// 0.27 -> 0.19.
 #include "cfr_vec.hpp"
 
 #include <type_traits>
@@ -327,6 +336,61 @@ __global__ void k_show_images(Dev d, int o, int msort, int K, uint16_t* out) {
     }
 }
 
+// ------------------------------------------------------------ chance nodes
+// Chance node without runout terminals (cfr.rs:637-663): per hand the sum of
+// its representatives' children in card order, times 1 / divisor.  One hand
+// per thread, `chunks` CTAs per node; the children's values are loaded sixteen
+// cards at a time and added in order (a skipped card adds +0, which changes
+// no bits of a sum that starts at +0).
+constexpr int kChanceThreads = 64, kChanceBatch = 16;
+__global__ void __launch_bounds__(kChanceThreads) kv_chance(Dev d, const ChanceItem* items, int p, uint32_t chunks) {
+    __shared__ CardEntry s_c[52 + kChanceBatch];
+    const uint32_t nd = blockIdx.x / chunks;
+    const ChanceItem c = items[nd];
+    for (uint32_t t = threadIdx.x; t < 52 + kChanceBatch; t += kChanceThreads)
+        s_c[t] = t < c.cc_count ? d.cards[c.cc_start + t] : CardEntry{0xFFu, 0, 0, 0};
+    __syncthreads();
+    const int nh = pick(d.nh, p), i = (int)((blockIdx.x - nd * chunks) * kChanceThreads + threadIdx.x);
+    if (i >= nh) return;
+    const uint64_t hm = pick(d.mask, p)[i];
+    const uint16_t* hp = pick(d.hperm, p);
+    float acc = 0.0f;
+    for (uint32_t t0 = 0; t0 < c.cc_count; t0 += kChanceBatch) {
+        float v[kChanceBatch];
+#pragma unroll
+        for (uint32_t j = 0; j < kChanceBatch; j++) {
+            const CardEntry e = s_c[t0 + j];
+            const uint32_t card = e.card & 0xFF;
+            v[j] = 0.0f;
+            if (card < 52u && !(hm >> card & 1ull)) {
+                const int src = e.perm ? (int)hp[(size_t)e.perm * nh + i] : i;
+                v[j] = d.cfv[(size_t)e.child_cslot * d.nh_max + src];
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kChanceBatch; j++) acc += v[j];
+    }
+    d.cfv[(size_t)c.cslot * d.nh_max + i] = acc * c.inv;
+}
+// Chance edges of player q: the parent's reach with the holders of the card
+// zeroed; a thread takes four hands of one edge.
+__global__ void __launch_bounds__(256) kv_edges(Dev d, const EdgeItem* items, uint32_t count, int q, uint32_t quads) {
+    const uint64_t g = (uint64_t)blockIdx.x * 256u + threadIdx.x;
+    const uint32_t e = (uint32_t)(g / quads), k = (uint32_t)(g - (uint64_t)e * quads);
+    if (e >= count) return;
+    const uint32_t card = items[e].card;
+    const size_t str = (size_t)pick(d.rstr, q);
+    float* base = pick(d.reach, q);
+    float4 v = ((const float4*)(base + (size_t)items[e].prs[q] * str))[k];
+    const uint4 h = ((const uint4*)pick(d.hinfo, q))[k];
+    auto keep = [&](uint32_t w) { return (w & 63u) != card && (w >> 6 & 63u) != card; };
+    if (!keep(h.x)) v.x = 0.0f;
+    if (!keep(h.y)) v.y = 0.0f;
+    if (!keep(h.z)) v.z = 0.0f;
+    if (!keep(h.w)) v.w = 0.0f;
+    ((float4*)(base + (size_t)items[e].crs[q] * str))[k] = v;
+}
+
 template <class F>
 bool with_show(const ShowShape& sh, F f) {
     auto by_k = [&](auto G, auto NT) {
@@ -382,6 +446,20 @@ void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s) {
         kv_show<G(), NT(), K()><<<sg.count, NT(), smem, s>>>(d, sg.items, (const uint16_t*)sg.img[o],
                                                              (const HandRank*)sg.ranks[p], p, sg.max_sorted[o]);
     });
+}
+void vec_chance(const Dev& d, const ChanceItem* items, uint32_t count, int p, cudaStream_t s) {
+    if (!count) return;
+    const uint32_t chunks = (uint32_t)((d.nh[p] + kChanceThreads - 1) / kChanceThreads);
+    kv_chance<<<count * chunks, kChanceThreads, 0, s>>>(d, items, p, chunks);
+}
+void vec_edges(const Dev& d, const EdgeItem* items, uint32_t count, int qmask, cudaStream_t s) {
+    if (!count) return;
+    for (int q = 0; q < 2; q++) {
+        if (!(qmask >> q & 1)) continue;
+        const uint32_t quads = (uint32_t)(d.rstr[q] / 4);
+        const uint64_t n = (uint64_t)count * quads;
+        kv_edges<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, items, count, q, quads);
+    }
 }
 
 }  // namespace gtob

@@ -45,5 +45,9 @@ size_t hand_rank_bytes();
 size_t show_image_bytes(const ShowShape& sh, int max_sorted);
 void build_show_tables(const Dev& d, const ShowGroups& sg, uint32_t slots, cudaStream_t s);
 void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s);
+// Chance nodes of one level (no runout terminals), and its chance edges' reach
+// for the players of qmask.
+void vec_chance(const Dev& d, const ChanceItem* items, uint32_t count, int p, cudaStream_t s);
+void vec_edges(const Dev& d, const EdgeItem* items, uint32_t count, int qmask, cudaStream_t s);
 
 }  // namespace gtob

@@ -384,6 +384,10 @@ struct EngineImpl {
     }
 
     void launch_chance(const Span& sc, int p) {
+        if (!plan.fused) {  // no runout terminals to evaluate in place
+            vec_chance(d, chance + sc.start, sc.count, p, stream);
+            return;
+        }
         // runout showdowns: f32 sums in the fused engine, f64 in the plain one
         if (plan.fused && !term64) k_chance<float><<<sc.count, kThreads, chance_smem, stream>>>(d, chance + sc.start, p);
         else k_chance<long long><<<sc.count, kThreads, chance_smem, stream>>>(d, chance + sc.start, p);
@@ -395,7 +399,9 @@ struct EngineImpl {
     // sweep computed it (that sweep's traverser was the other player), so its
     // slots still hold exactly the values a full recomputation would write.
     void down(int qmask, int mode, Profile* pr) {
-        timed(pr, 0, [&] { k_copy_root<<<4, kThreads, 0, stream>>>(d); });
+        // the root slots keep the ranges' weights once a full sweep has written
+        // them; the profile still times the copy
+        if (pr || qmask == 3) timed(pr, 0, [&] { k_copy_root<<<4, kThreads, 0, stream>>>(d); });
         const int L = plan.num_levels;
         for (int l = 0; l < L; l++) {
             if (use_river()) {  // two runs when both players' reach is refreshed
@@ -410,7 +416,10 @@ struct EngineImpl {
             }
             const Span se = plan.edge_span[l];
             if (se.count)
-                timed(pr, 2, [&] { k_down_chance<<<se.count, kThreads, 0, stream>>>(d, edge + se.start, qmask); });
+                timed(pr, 2, [&] {
+                    if (vec) vec_edges(d, edge + se.start, se.count, qmask, stream);
+                    else k_down_chance<<<se.count, kThreads, 0, stream>>>(d, edge + se.start, qmask);
+                });
         }
     }
     // Before the first CFR sweep after anything else wrote the reach slots
