@@ -59,6 +59,7 @@ struct Dev {
     unsigned* err;  // device error bits (bounded waits that gave up, bad copies)
     // staged engine extras
     const uint32_t* hinfo[2];   // per hand: c1 | c2 << 6 | same << 16 (0xFFFF: no same combo)
+    const struct FoldSum* folds;  // the sweep's fold summaries (vector kernels)
     const uint32_t* node_id[2];  // tree node id of each device action node (per player, by sidx)
     // river programs: per player o, the showdown table images of every river
     // board (river_tab_words words each) and their word offsets (num_slots + 1)
@@ -211,11 +212,17 @@ template <int KA>
 struct alignas(16) SNodeT {
     uint64_t aoff;             // arena offset (elements) in the actor's arena
     uint32_t cslot, rslot, oslot, sidx;
-    uint32_t cs[KA];           // child cfv slots (kNoSlot: the fold child)
+    uint32_t cs[KA];           // child cfv slots (the fold child: its fold's number)
     uint32_t rs[KA];           // child reach slots of the actor (down sweep; kNoSlot: none)
     uint32_t actor, na, fk;    // fk: the fold child's index, kNoSlot if none
     uint32_t folder;           // the folding player of the fold child
     float twin, tlose;         // fold payoffs
+};
+// One fold's opponent reach vector, summarised (game.rs:478-485) with exact
+// sums: per card, in total, and the grid scale they are on.
+struct alignas(16) FoldSum {
+    long long S[52], T;
+    int sc, pad;
 };
 using SNode = SNodeT<kSKA>;
 static_assert(sizeof(SNode) == 80 && sizeof(SNodeT<kVKA>) == 112, "SNode layout");

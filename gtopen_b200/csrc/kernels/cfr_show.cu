@@ -232,6 +232,29 @@ __device__ __forceinline__ void show_group(const Dev& d, unsigned char* sm, cons
     }
 }
 
+// A vector of a batch of G into the interleaved rows r[hand * G + g] (g the
+// thread's vector), four hands a load; returns the largest value's bits over
+// this thread's hands.
+template <int G, int NT>
+__device__ __forceinline__ uint32_t stage_interleaved(const float* src, bool live, int nho, int nho_pad, float* r) {
+    const int q4 = nho_pad >> 2, tid = (int)threadIdx.x, g = tid & (G - 1);
+    uint32_t mx = 0u;
+    for (int q = tid / G; q < q4; q += NT / G) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (live) v = ((const float4*)src)[q];
+        const float x[4] = {v.x, 4 * q + 1 < nho ? v.y : 0.0f, 4 * q + 2 < nho ? v.z : 0.0f,
+                            4 * q + 3 < nho ? v.w : 0.0f};
+        mx = max(mx, __float_as_uint(fmaxf(fmaxf(fmaxf(x[0], 0.0f), x[1]), fmaxf(fmaxf(x[2], 0.0f), x[3]))));
+#pragma unroll
+        for (int j = 0; j < 4; j++) {  // rotated so that the warp's quads write different banks
+            const int k = (j + q) & 3;
+            const float y = k == 0 ? x[0] : k == 1 ? x[1] : k == 2 ? x[2] : x[3];
+            r[(4 * q + k) * G + g] = y;
+        }
+    }
+    return mx;
+}
+
 template <int G, int NT, int K>
 __global__ void __launch_bounds__(NT) kv_show(Dev d, const ShowItem* items, const uint16_t* img, const HandRank* ranks,
                                               int p, int msort) {
@@ -257,26 +280,8 @@ __global__ void __launch_bounds__(NT) kv_show(Dev d, const ShowItem* items, cons
         uint4* im = (uint4*)(sm + SL.o_img);
         for (int k = tid; k < il / 8; k += NT) im[k] = src[k];
     }
-    uint32_t mx = 0u;
-    {  // the reach vectors, interleaved by showdown: four hands a load
-        const int q4 = nho_pad >> 2;
-        const bool live = it.cslot != kNoSlot;
-        const float* src = pick(d.reach, o) + (size_t)it.rs[o] * pick(d.rstr, o);
-        float* r = (float*)(sm + SL.o_r);
-        for (int q = tid / G; q < q4; q += NT / G) {
-            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (live) v = ((const float4*)src)[q];
-            const float x[4] = {v.x, 4 * q + 1 < nho ? v.y : 0.0f, 4 * q + 2 < nho ? v.z : 0.0f,
-                                4 * q + 3 < nho ? v.w : 0.0f};
-            mx = max(mx, __float_as_uint(fmaxf(fmaxf(fmaxf(x[0], 0.0f), x[1]), fmaxf(fmaxf(x[2], 0.0f), x[3]))));
-#pragma unroll
-            for (int j = 0; j < 4; j++) {  // rotated so that the warp's quads write different banks
-                const int k = (j + q) & 3;
-                const float y = k == 0 ? x[0] : k == 1 ? x[1] : k == 2 ? x[2] : x[3];
-                r[(4 * q + k) * G + g] = y;
-            }
-        }
-    }
+    uint32_t mx = stage_interleaved<G, NT>(pick(d.reach, o) + (size_t)it.rs[o] * pick(d.rstr, o), it.cslot != kNoSlot, nho,
+                                           nho_pad, (float*)(sm + SL.o_r));
 #pragma unroll
     for (int x = G; x < 32; x <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, x));
     __syncthreads();
@@ -290,6 +295,82 @@ __global__ void __launch_bounds__(NT) kv_show(Dev d, const ShowItem* items, cons
         show_group<G, NT, K, true>(d, sm, SL, s_it, s_w, s_wf, ga, gb, m, nhp, hr, pick(d.hinfo, p));
     else
         show_group<G, NT, K, false>(d, sm, SL, s_it, s_w, s_wf, ga, gb, m, nhp, hr, pick(d.hinfo, p));
+}
+
+// ------------------------------------------------------------------- folds
+// The sweep's fold summaries: G folds a CTA, their opponent vectors
+// interleaved as in kv_show, a lane per card list and pair of folds.  Every
+// fold of a player uses the same card lists, so a row of the interleaved
+// vectors serves all of them.  Inside the up kernels these sums took three
+// block barriers and a third of the traverser's instructions per node; as one
+// launch beside the showdowns the opponent's nodes and f32 updates need no
+// barrier at all.  470 v 647 hands, 85,413 folds: 0.13 ms a sweep (issue 74%
+// of peak, the conversions 52%).  One iteration before -> after: that flop,
+// 16-bit, 3.9 -> 3.7 ms; turn f32 0.364 -> 0.291; river f32 0.072 -> 0.058.
+constexpr int kFoldThreads = 256;
+// folds per CTA: short lists leave a CTA of 8 with more set-up than sums
+inline int fold_group(int nho) { return nho <= 128 ? 32 : 8; }
+template <int G>
+__global__ void __launch_bounds__(kFoldThreads) kv_folds(Dev d, const uint32_t* slots, uint32_t count, int p,
+                                                         FoldSum* out) {
+    constexpr int L = G / 2, NC = kFoldThreads / L;
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ uint32_t s_mx[G];
+    __shared__ longlong2 s_S[52 * L];
+    const int o = 1 - p, nho = pick(d.nh, o), nho_pad = (nho + 3) & ~3;
+    const int tid = (int)threadIdx.x, g = tid & (G - 1);
+    const uint32_t f0 = blockIdx.x * G, fg = f0 + (uint32_t)g;
+    if (tid < G) s_mx[tid] = 0u;
+    const float* src = pick(d.reach, o) + (size_t)(fg < count ? slots[fg] : 0u) * pick(d.rstr, o);
+    uint32_t mx = stage_interleaved<G, kFoldThreads>(src, fg < count, nho, nho_pad, (float*)sm);
+#pragma unroll
+    for (int x = G; x < 32; x <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+    __syncthreads();
+    if ((tid & 31) < G) atomicMax(&s_mx[g], mx);
+    __syncthreads();
+    const int l = tid & (L - 1), c_ = tid / L;
+    const Grid ga = make_grid(__uint_as_float(s_mx[2 * l])), gb = make_grid(__uint_as_float(s_mx[2 * l + 1]));
+    const uint32_t fa = f0 + 2 * (uint32_t)l;
+    const bool onA = fa < count, onB = fa + 1 < count;
+    const uint16_t* idx = pick(d.hcard_idx, o);
+    for (int c = c_; c < 52; c += NC) {
+        const uint32_t b = pick(d.hcard_off, o)[c], e = pick(d.hcard_off, o)[c + 1];
+        const float2* r2 = (const float2*)sm + l;
+        longlong2 a = make_longlong2(0, 0);
+        const bool big = ga.S > 126 || gb.S > 126;
+#pragma unroll 4
+        for (uint32_t k = b; k < e; k++) {
+            const float2 x = r2[(int)idx[k] * L];
+            a.x += big ? grid_q<true>(ga, x.x) : grid_q<false>(ga, x.x);
+            a.y += big ? grid_q<true>(gb, x.y) : grid_q<false>(gb, x.y);
+        }
+        s_S[c * L + l] = a;
+        if (onA) out[fa].S[c] = a.x;
+        if (onB) out[fa + 1].S[c] = a.y;
+    }
+    __syncthreads();
+    if (tid < 32) {  // every hand holds two cards: the total is half the card sums' sum
+        longlong2 t = make_longlong2(0, 0);
+        for (int k = c_; k < 52; k += 32 / L) {
+            t.x += s_S[k * L + l].x;
+            t.y += s_S[k * L + l].y;
+        }
+#pragma unroll
+        for (int x = L; x < 32; x <<= 1) {
+            t.x += __shfl_xor_sync(0xffffffffu, t.x, x);
+            t.y += __shfl_xor_sync(0xffffffffu, t.y, x);
+        }
+        if (tid < L) {
+            if (onA) {
+                out[fa].T = t.x >> 1;
+                out[fa].sc = ga.S;
+            }
+            if (onB) {
+                out[fa + 1].T = t.y >> 1;
+                out[fa + 1].sc = gb.S;
+            }
+        }
+    }
 }
 
 // The boards' rank entries by hand, for kv_show (once per engine).
@@ -446,6 +527,20 @@ void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s) {
         kv_show<G(), NT(), K()><<<sg.count, NT(), smem, s>>>(d, sg.items, (const uint16_t*)sg.img[o],
                                                              (const HandRank*)sg.ranks[p], p, sg.max_sorted[o]);
     });
+}
+size_t fold_sum_bytes() { return sizeof(FoldSum); }
+const void* fold_kernel(size_t* smem, int nho) {
+    const int G = fold_group(nho);
+    *smem = (size_t)((nho + 3) & ~3) * G * 4;
+    return G == 8 ? (const void*)kv_folds<8> : (const void*)kv_folds<32>;
+}
+void vec_folds(const Dev& d, const uint32_t* slots, uint32_t count, int p, cudaStream_t s) {
+    if (!count) return;
+    const int nho = d.nh[1 - p], G = fold_group(nho);
+    const unsigned grid = (count + G - 1) / G, smem = (unsigned)((nho + 3) & ~3) * G * 4;
+    FoldSum* out = const_cast<FoldSum*>(d.folds);
+    if (G == 8) kv_folds<8><<<grid, kFoldThreads, smem, s>>>(d, slots, count, p, out);
+    else kv_folds<32><<<grid, kFoldThreads, smem, s>>>(d, slots, count, p, out);
 }
 void vec_chance(const Dev& d, const ChanceItem* items, uint32_t count, int p, cudaStream_t s) {
     if (!count) return;

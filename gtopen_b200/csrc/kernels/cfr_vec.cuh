@@ -5,19 +5,23 @@
 // registers: arena blocks are hand-major ([hand * na + action]), so its
 // entries are V * na consecutive elements, read and written with the widest
 // aligned loads, and hand vectors (reach, child values) are read V floats at
-// a time.  Nothing is staged in shared memory, and the only block-wide steps
-// are the node's maxima (quantised arenas) and the fold child's card sums.
+// a time.  Nothing is staged in shared memory, and the only block-wide step is
+// the node's maxima in the update of quantised arenas: a fold child's card
+// sums come from the sweep's fold summaries (cfr_show.cu).
 //
 // What bounds them, and why this split: the bulk-copy kernels they replace
 // kept each node's blocks in shared memory and touched every 16-bit entry
 // with two-byte shared accesses, and a 128-thread CTA per node cost ~4.2 ns
 // of the device whatever its size.  Here
-//   * a node of up to 32 V hands is one warp, four nodes per CTA, no block
-//     barriers (V = 1, 2 or 4: the smallest that fits, so that a node of 24
-//     hands costs one hand's instructions per lane);
-//   * a larger node is one CTA of ceil(hands / 128) warps (V = 4: half the
-//     warps, and half their per-warp work, of V = 2 -- 1.52 against 2.35 ms
-//     for the traverser's nodes of a 470 v 647 flop).
+//   * where a node's hands do not depend on one another -- the down sweep,
+//     the opponent's nodes, evaluation sweeps, f32 updates -- a warp takes
+//     32 V hands of one node, no barriers; V = 4 fills a load (470 v 647
+//     hands: down 0.45 ms, V = 2 0.57, V = 1 0.69), V = 1 or 2 where the node
+//     is smaller or the launch too small to fill the device;
+//   * the update of quantised arenas takes the node's maxima first: a node of
+//     up to 128 hands is one warp, a larger one a CTA of ceil(hands / 128)
+//     warps (V = 4: half the warps, and half their per-warp work, of V = 2 --
+//     1.52 against 2.35 ms for the traverser's nodes of a 470 v 647 flop).
 // One iteration with only this changed, B200, bulk-copy kernels before ->
 // after: flop of 284,901 nodes at 28 v 23 hands, f32 1.83 -> 1.05 ms; flop of
 // 609,894 nodes at 64 v 39, 16-bit 3.58 -> 2.02 ms; flop of 346,255 nodes at
@@ -38,10 +42,8 @@
 namespace gtob {
 namespace {
 
-constexpr int kVWarpNodes = 4;  // nodes per CTA of the warp-per-node form
 constexpr int kVMaxWarps = 32;
-constexpr int kVCta = 4;  // hands per thread of the CTA-per-node form
-constexpr int kVCtaThreads = (1326 + 32 * kVCta - 1) / (32 * kVCta) * 32;
+constexpr uint64_t kVFillWarps = 148 * 16;  // warps that fill the device
 
 // ------------------------------------------------------- register vectors
 template <int B> struct Gran;
@@ -87,31 +89,11 @@ union Pack {
 template <class T>
 __device__ __forceinline__ T pick(T const (&x)[2], int a) { return a ? x[1] : x[0]; }
 
-template <bool WARP>
-__device__ __forceinline__ void gsync() {
-    if (WARP) __syncwarp();
-    else __syncthreads();
-}
 // The thread's place in its node, and the node's scratch in shared memory.
 struct Group {
-    int t, W;           // thread within the node, warps of the node
-    long long* S;       // 52 card sums
-    long long* q;       // opponent hands' grid values
-    float* r;           // the opponent reach they came from
-    uint32_t* red;      // 3 * kVMaxWarps
+    int t, W;       // thread within the node, warps of the node
+    uint32_t* red;  // 3 * kVMaxWarps
 };
-constexpr unsigned kVHead = 52 * 8 + 3 * kVMaxWarps * 4;
-__host__ __device__ inline unsigned group_bytes(int nh_pad) { return kVHead + (unsigned)nh_pad * 12u; }
-__device__ __forceinline__ Group make_group(unsigned char* sm, int nh_pad, int t, int W) {
-    Group g;
-    g.t = t;
-    g.W = W;
-    g.S = (long long*)sm;
-    g.red = (uint32_t*)(sm + 52 * 8);
-    g.q = (long long*)(sm + kVHead);
-    g.r = (float*)(g.q + nh_pad);
-    return g;
-}
 // Maxima of non-negative floats over the node's threads (their bits order as
 // unsigned integers): one redux per value and warp, one barrier.
 template <bool WARP, int N>
@@ -294,106 +276,58 @@ __global__ void __launch_bounds__(128) kv_down(Dev d, Arenas ar, const SNodeT<KA
 }
 
 // --------------------------------------------------------------- up sweep
-// The fold child's summary (game.rs:478-485), exact sums: the opponent
-// vector's scale, every hand's grid value in shared memory, the 52 card sums
-// from the hands' card lists (four threads a card), the total as half the
-// card sums' sum (every hand holds two cards).  Three barriers.
-template <bool WARP, int V>
-__device__ __forceinline__ long long v_fold_sums(const Dev& d, int o, const float* ro, const Group& g, int& sc) {
-    const int nho = pick(d.nh, o), lane = threadIdx.x & 31, step = g.W * 32 * V;
-    Pack<float, V> r;
-    float mx[1] = {0.0f};
-    for (int j = g.t * V; j < nho; j += step) {
-        r.load(ro + j);
-        if (nho - j < V) r.keep(nho - j);
+// The node's child values for this thread's hands: rows of cfv, and the fold
+// child's value from its fold's summary (game.rs:487-496).
+template <int NA, int V, class NODE>
+__device__ __forceinline__ void v_children(const Dev& d, const NODE& it, int p, int i0, Pack<float, V> (&cv)[NA]) {
+    const int nh = pick(d.nh, p), live = nh - i0, fk = (int)it.fk;
+    if (live <= 0) {
 #pragma unroll
-        for (int u = 0; u < V; u++) mx[0] = fmaxf(mx[0], r.e[u]);
-        r.store(g.r + j);
+        for (int k = 0; k < NA; k++) cv[k].zero();
+        return;
     }
-    group_max<WARP>(g, mx);
-    sc = fix_scale(mx[0]);
-    for (int j = g.t * V; j < nho; j += step) {  // (the thread's own entries of g.r)
-        r.load(g.r + j);
-#pragma unroll
-        for (int u = 0; u < V; u++) g.q[j + u] = fix_q(r.e[u], sc);
-    }
-    gsync<WARP>();
-    const uint32_t* off = pick(d.hcard_off, o);
-    const uint16_t* idx = pick(d.hcard_idx, o);
-    if (WARP) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int c = lane + 32 * h;
-            if (c < 52) {
-                long long s = 0;
-                const uint32_t e = off[c + 1];
-#pragma unroll 4
-                for (uint32_t k = off[c]; k < e; k++) s += g.q[idx[k]];
-                g.S[c] = s;
-            }
-        }
-    } else {
-        for (int w0 = g.t & ~31; w0 < 208; w0 += g.W * 32) {  // warp-uniform trip count
-            const int sl = w0 + lane, c = sl >> 2;
-            long long s = 0;
-            if (c < 52) {
-                const uint32_t e = off[c + 1];
-#pragma unroll 4
-                for (uint32_t k = off[c] + (sl & 3); k < e; k += 4) s += g.q[idx[k]];
-            }
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            if (c < 52 && (sl & 3) == 0) g.S[c] = s;
-        }
-    }
-    gsync<WARP>();
-    long long t = g.S[lane] + (lane < 20 ? g.S[32 + lane] : 0);
-#pragma unroll
-    for (int x = 16; x > 0; x >>= 1) t += __shfl_xor_sync(0xffffffffu, t, x);
-    return t >> 1;
-}
-// The node's child values for this thread's hands: staged rows, and the fold
-// child's value in place (game.rs:487-496).
-template <bool WARP, int NA, int V, class NODE>
-__device__ __forceinline__ void v_children(const Dev& d, const NODE& it, int p, const float* fold_ro, const Group& g,
-                                           Pack<float, V> (&cv)[NA]) {
-    const int nh = pick(d.nh, p), i0 = g.t * V, live = nh - i0, fk = (int)it.fk;
+    uint32_t fold = 0, frs = 0;
 #pragma unroll
     for (int k = 0; k < NA; k++) {
-        if (k == fk || live <= 0) cv[k].zero();
-        else cv[k].load(d.cfv + (size_t)it.cs[k] * d.nh_max + i0);
+        if (k == fk) {
+            cv[k].zero();
+            fold = it.cs[k];
+            frs = it.rs[k];
+        } else {
+            cv[k].load(d.cfv + (size_t)it.cs[k] * d.nh_max + i0);
+        }
     }
-    if (live > 0 && live < V) {
+    if (live < V) {
 #pragma unroll
         for (int k = 0; k < NA; k++) cv[k].keep(live);
     }
     if (fk < 0) return;
-    int sc;
-    const long long total = v_fold_sums<WARP, V>(d, 1 - p, fold_ro, g, sc);
+    // the folding player's reach was written by the down sweep at an
+    // opponent's node; at the traverser's it is the opponent's at the node
+    const int o = 1 - p;
+    const float* ro = pick(d.reach, o) + (size_t)((int)it.actor == p ? it.oslot : frs) * pick(d.rstr, o);
+    const FoldSum* fs = d.folds + fold;
+    const long long T = fs->T;
+    const int sc = fs->sc;
     const float amount = (int)it.folder == p ? it.tlose : it.twin;
+    Pack<uint32_t, V> hi;  // hand words are padded to whole groups of four
+    hi.load(pick(d.hinfo, p) + i0);
 #pragma unroll
     for (int u = 0; u < V; u++)
         if (u < live) {
-            const uint32_t h = pick(d.hinfo, p)[i0 + u], sm = h >> 16;
-            const float same_r = sm != 0xFFFFu ? g.r[sm] : 0.0f;
-            const float f = amount * (fix_f(total - g.S[h & 63u] - g.S[(h >> 6) & 63u], sc) + same_r);
+            const uint32_t h = hi.e[u], sm = h >> 16;
+            const float same_r = sm != 0xFFFFu ? ro[sm] : 0.0f;
+            const float f = amount * (fix_f(T - fs->S[h & 63u] - fs->S[(h >> 6) & 63u], sc) + same_r);
 #pragma unroll
             for (int k = 0; k < NA; k++)
                 if (k == fk) cv[k].e[u] = f;
         }
 }
-template <bool WARP, int NA, int V, class NODE>
-__device__ __forceinline__ void v_opp_node(const Dev& d, const NODE& it, int p, const Group& g) {
-    const int o = 1 - p, i0 = g.t * V;
-    Pack<float, V> cv[NA];
-    // the folding player's reach was written by the down sweep
-    uint32_t fr = 0;
-#pragma unroll
-    for (int k = 0; k < NA; k++)
-        if (k == (int)it.fk) fr = it.rs[k];
-    const float* ro = pick(d.reach, o) + (size_t)fr * pick(d.rstr, o);
-    v_children<WARP, NA, V>(d, it, p, ro, g, cv);
+template <int NA, int V, class NODE>
+__device__ __forceinline__ void v_opp_node(const Dev& d, const NODE& it, int p, int i0) {
     if (i0 >= pick(d.nh, p)) return;
+    Pack<float, V> cv[NA];
+    v_children<NA, V>(d, it, p, i0, cv);
     Pack<float, V> out;
 #pragma unroll
     for (int u = 0; u < V; u++) {
@@ -408,12 +342,12 @@ __device__ __forceinline__ void v_opp_node(const Dev& d, const NODE& it, int p, 
 // (best_response.rs:69-121, 185-219), or the CFR update (cfr.rs:297-409) with
 // the blocks and scales written back.
 template <int FMT, int EVAL, bool PRED, bool WARP, int NA, int V, class NODE>
-__device__ __forceinline__ void v_mine_node(const Dev& d, const Arenas& ar, const NODE& it, int p, int mode,
+__device__ __forceinline__ void v_mine_node(const Dev& d, const Arenas& ar, const NODE& it, int p, int mode, int i0,
                                             const Group& g) {
     using Q = QT<FMT == kDevFP8 ? kDevFP8 : kDevI16>;
     using QR = std::conditional_t<FMT == kDevF32, float, typename Q::R>;
     using QS = std::conditional_t<FMT == kDevF32, float, typename Q::S>;
-    const int o = 1 - p, nh = pick(d.nh, p), i0 = g.t * V, live = nh - i0;
+    const int nh = pick(d.nh, p), live = nh - i0;
     const bool on = live > 0;
     const size_t e0 = it.aoff + (size_t)i0 * NA;
     const long long loff = pick(d.lock_off, p)[it.sidx];
@@ -447,7 +381,7 @@ __device__ __forceinline__ void v_mine_node(const Dev& d, const Arenas& ar, cons
         rp.keep(live);
     }
     Pack<float, V> cv[NA], out;
-    v_children<WARP, NA, V>(d, it, p, pick(d.reach, o) + (size_t)it.oslot * pick(d.rstr, o), g, cv);
+    v_children<NA, V>(d, it, p, i0, cv);
     float* outp = d.cfv + (size_t)it.cslot * d.nh_max + i0;
     if (loff >= 0 || EVAL) {
         if (!on) return;
@@ -576,105 +510,134 @@ __device__ __forceinline__ void v_mine_node(const Dev& d, const Arenas& ar, cons
     }
 }
 
-#define V_GROUP()                                                                                      \
-    extern __shared__ __align__(16) unsigned char sm[];                                                \
-    const int w_ = (int)(threadIdx.x >> 5);                                                            \
-    const uint32_t n = WARP ? blockIdx.x * kVWarpNodes + w_ : blockIdx.x;                              \
-    if (n >= count) return;                                                                            \
-    const SNodeT<KA>& it = nodes[n];                                                                  \
-    const Group g = WARP ? make_group(sm + (size_t)w_ * group_bytes(d.nh_pad), d.nh_pad,               \
-                                      (int)(threadIdx.x & 31), 1)                                      \
-                         : make_group(sm, d.nh_pad, (int)threadIdx.x, (int)(blockDim.x >> 5));
-
-template <bool WARP, int V, int KA>
-__global__ void __launch_bounds__(WARP ? 32 * kVWarpNodes : kVCtaThreads) kv_up_opp(Dev d, const SNodeT<KA>* nodes, uint32_t count, int p) {
-    V_GROUP()
+// Nodes whose hands do not depend on one another (the opponent's nodes,
+// evaluation sweeps, f32 arenas): one warp per 32 V hands, wn warps per node.
+template <int V, int KA>
+__global__ void __launch_bounds__(128) kv_up_opp(Dev d, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn, int p) {
+    const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
+    if (n >= count) return;
+    const SNodeT<KA>& it = nodes[n];
+    const int i0 = (int)((w - n * wn) * 32 + (threadIdx.x & 31)) * V;
 #undef V_CASE
-#define V_CASE(NA)                                                                   \
-    case NA:                                                                         \
-        if (NA <= KA) v_opp_node<WARP, NA <= KA ? NA : 1, V>(d, it, p, g);           \
+#define V_CASE(NA)                                                    \
+    case NA:                                                          \
+        if (NA <= KA) v_opp_node<NA <= KA ? NA : 1, V>(d, it, p, i0); \
         break;
     switch (it.na) {
         V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
     }
 }
-template <int FMT, int EVAL, bool PRED, bool WARP, int V, int KA>
-__global__ void __launch_bounds__(WARP ? 32 * kVWarpNodes : kVCtaThreads) kv_up_mine(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, int p,
-                                                  int mode) {
-    V_GROUP()
+template <int FMT, int EVAL, bool PRED, int V, int KA>
+__global__ void __launch_bounds__(128) kv_up_mine(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn,
+                                                  int p, int mode) {
+    static_assert(EVAL || FMT == kDevF32, "a quantised update needs the node's maxima");
+    const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
+    if (n >= count) return;
+    const SNodeT<KA>& it = nodes[n];
+    const int i0 = (int)((w - n * wn) * 32 + (threadIdx.x & 31)) * V;
 #undef V_CASE
-#define V_CASE(NA)                                                                                          \
-    case NA:                                                                                                \
-        if (NA <= KA) v_mine_node<FMT, EVAL, PRED, WARP, NA <= KA ? NA : 1, V>(d, ar, it, p, mode, g);       \
+#define V_CASE(NA)                                                                                               \
+    case NA:                                                                                                     \
+        if (NA <= KA) v_mine_node<FMT, EVAL, PRED, true, NA <= KA ? NA : 1, V>(d, ar, it, p, mode, i0, Group{}); \
+        break;
+    switch (it.na) {
+        V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
+    }
+}
+// Updates of quantised arenas: one warp per node (WARP), or one CTA.
+template <int FMT, bool PRED, bool WARP, int V, int KA>
+__global__ void __launch_bounds__(WARP ? 128 : (1326 + 32 * V - 1) / (32 * V) * 32)
+    kv_up_quant(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, int p) {
+    __shared__ uint32_t red[WARP ? 1 : 3 * kVMaxWarps];
+    const uint32_t n = WARP ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
+    if (n >= count) return;
+    const SNodeT<KA>& it = nodes[n];
+    const Group g{(int)(WARP ? threadIdx.x & 31 : threadIdx.x), (int)(blockDim.x >> 5), red};
+#undef V_CASE
+#define V_CASE(NA)                                                                                        \
+    case NA:                                                                                              \
+        if (NA <= KA) v_mine_node<FMT, 0, PRED, WARP, NA <= KA ? NA : 1, V>(d, ar, it, p, 0, g.t * V, g); \
         break;
     switch (it.na) {
         V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
     }
 }
 
-// The form of a launch for traverser p: f(warp form, V).  The warp form also
-// keeps four nodes' opponent vectors in the default shared memory.
+template <int N>
+using IntC = std::integral_constant<int, N>;
+// Hands per lane of the forms whose warps are independent: four, unless the
+// node is smaller, or the launch too small to fill the device with warps of
+// 128 hands -- then fewer hands a lane shorten the one wave there is.
+inline int lane_hands(int nh, uint32_t count) {
+    if (nh <= 32) return 1;
+    const uint64_t w4 = (uint64_t)count * (uint32_t)((nh + 127) / 128);
+    if (w4 <= kVFillWarps / 4) return 1;
+    if (nh <= 64 || w4 <= kVFillWarps / 2) return 2;
+    return 4;
+}
+// f(V, warps per node, grid) for a launch of count nodes of nh hands
 template <class F>
-void with_shape(const Dev& d, int p, F f) {
-    const int nh = d.nh_pad <= 512 ? d.nh[p] : 1326;
-    if (nh <= 32) f(std::true_type{}, std::integral_constant<int, 1>{});
-    else if (nh <= 64) f(std::true_type{}, std::integral_constant<int, 2>{});
-    else if (nh <= 128) f(std::true_type{}, std::integral_constant<int, 4>{});
-    else f(std::false_type{}, std::integral_constant<int, kVCta>{});
-}
-struct Shape {
-    dim3 grid;
-    unsigned block, smem;
-};
-template <bool WARP, int V>
-Shape up_shape(const Dev& d, uint32_t count, int nh) {
-    const unsigned gb = group_bytes(d.nh_pad);
-    if (WARP) return {dim3((count + kVWarpNodes - 1) / kVWarpNodes), 32u * kVWarpNodes, gb * kVWarpNodes};
-    return {dim3(count), (unsigned)((nh + 32 * V - 1) / (32 * V)) * 32u, gb};
+void with_lanes(int nh, uint32_t count, F f) {
+    auto go = [&](auto V) {
+        const uint32_t wn = (uint32_t)((nh + 32 * V() - 1) / (32 * V()));
+        f(V, wn, (unsigned)(((uint64_t)count * wn + 3) / 4));
+    };
+    const int v = lane_hands(nh, count);
+    if (v == 1) go(IntC<1>{});
+    else if (v == 2) go(IntC<2>{});
+    else go(IntC<4>{});
 }
 
 // The launches of one arena format.
 template <int FMT, int KA>
 void down_t(const Dev& d, const Arenas& ar, const VecNodes& n, int nh, int mode, cudaStream_t s) {
     const auto* nodes = (const SNodeT<KA>*)n.nodes;
-    auto go = [&](auto S, auto V) {
-        const uint32_t wn = (uint32_t)((nh + 32 * V() - 1) / (32 * V()));
-        const uint64_t warps = (uint64_t)n.count * wn;
-        kv_down<FMT, S(), V(), KA><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(d, ar, nodes, n.count, wn);
-    };
-    auto by_v = [&](auto S) {
-        if (FMT == kDevFP8) go(S, std::integral_constant<int, 4>{});
-        else if (nh <= 32) go(S, std::integral_constant<int, FMT == kDevFP8 ? 4 : 1>{});
-        else if (nh <= 64) go(S, std::integral_constant<int, FMT == kDevFP8 ? 4 : 2>{});
-        else go(S, std::integral_constant<int, 4>{});
-    };
-    if (mode) by_v(std::integral_constant<int, kVAverage>{});
-    else if (ar.pred[0]) by_v(std::integral_constant<int, kVPredicted>{});
-    else by_v(std::integral_constant<int, kVRegret>{});
+    with_lanes(nh, n.count, [&](auto V, uint32_t wn, unsigned grid) {
+        constexpr int v = V();
+        if (mode) kv_down<FMT, kVAverage, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn);
+        else if (ar.pred[0]) kv_down<FMT, kVPredicted, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn);
+        else kv_down<FMT, kVRegret, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn);
+    });
 }
 template <int FMT, int KA>
 void up_mine_t(const Dev& d, const Arenas& ar, const VecNodes& n, int p, int eval, cudaStream_t s) {
     const auto* nodes = (const SNodeT<KA>*)n.nodes;
-    auto go = [&](auto WP, auto V) {
-        constexpr bool W = WP();
-        const Shape sh = up_shape<W, V()>(d, n.count, d.nh[p]);
-        if (eval >= 0)
-            kv_up_mine<FMT, 1, false, W, V(), KA><<<sh.grid, sh.block, sh.smem, s>>>(d, ar, nodes, n.count, p, eval);
-        else if (ar.pred[0])
-            kv_up_mine<FMT, 0, true, W, V(), KA><<<sh.grid, sh.block, sh.smem, s>>>(d, ar, nodes, n.count, p, 0);
-        else
-            kv_up_mine<FMT, 0, false, W, V(), KA><<<sh.grid, sh.block, sh.smem, s>>>(d, ar, nodes, n.count, p, 0);
-    };
-    // FP8 (the precision study's format) keeps to the form that takes any hand count
-    if constexpr (FMT == kDevFP8) go(std::false_type{}, std::integral_constant<int, kVCta>{});
-    else with_shape(d, p, go);
+    const int nh = d.nh[p];
+    if (eval >= 0 || FMT == kDevF32) {
+        with_lanes(nh, n.count, [&](auto V, uint32_t wn, unsigned grid) {
+            constexpr int v = V();
+            if (eval >= 0) {
+                kv_up_mine<FMT, 1, false, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn, p, eval);
+            } else if constexpr (FMT == kDevF32) {
+                if (ar.pred[0]) kv_up_mine<FMT, 0, true, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn, p, 0);
+                else kv_up_mine<FMT, 0, false, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn, p, 0);
+            }
+        });
+        return;
+    }
+    if constexpr (FMT != kDevF32) {
+        auto go = [&](auto WP, auto V) {
+            constexpr bool W = WP();
+            constexpr int v = V();
+            const unsigned grid = W ? (n.count + 3) / 4 : n.count;
+            const unsigned block = W ? 128u : (unsigned)((nh + 32 * v - 1) / (32 * v)) * 32u;
+            if (ar.pred[0]) kv_up_quant<FMT, true, W, v, KA><<<grid, block, 0, s>>>(d, ar, nodes, n.count, p);
+            else kv_up_quant<FMT, false, W, v, KA><<<grid, block, 0, s>>>(d, ar, nodes, n.count, p);
+        };
+        // small launches: a CTA per node with fewer hands a thread
+        const bool small = (uint64_t)n.count * (uint32_t)((nh + 127) / 128) <= kVFillWarps / 2;
+        if (nh <= 32) go(std::true_type{}, IntC<1>{});
+        else if (nh <= 64) go(std::true_type{}, IntC<2>{});
+        else if (nh <= 128 && !small) go(std::true_type{}, IntC<4>{});
+        else if (small) go(std::false_type{}, IntC<2>{});
+        else go(std::false_type{}, IntC<4>{});
+    }
 }
 template <int KA>
 void up_opp_t(const Dev& d, const VecNodes& n, int p, cudaStream_t s) {
-    with_shape(d, p, [&](auto WP, auto V) {
-        constexpr bool W = WP();
-        const Shape sh = up_shape<W, V()>(d, n.count, d.nh[p]);
-        kv_up_opp<W, V(), KA><<<sh.grid, sh.block, sh.smem, s>>>(d, (const SNodeT<KA>*)n.nodes, n.count, p);
+    with_lanes(d.nh[p], n.count, [&](auto V, uint32_t wn, unsigned grid) {
+        constexpr int v = V();
+        kv_up_opp<v, KA><<<grid, 128, 0, s>>>(d, (const SNodeT<KA>*)n.nodes, n.count, wn, p);
     });
 }
 }  // namespace

@@ -45,6 +45,11 @@ size_t hand_rank_bytes();
 size_t show_image_bytes(const ShowShape& sh, int max_sorted);
 void build_show_tables(const Dev& d, const ShowGroups& sg, uint32_t slots, cudaStream_t s);
 void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s);
+// A sweep's fold summaries into d.folds: fold k's opponent vector is reach
+// slot slots[k].
+size_t fold_sum_bytes();
+const void* fold_kernel(size_t* smem, int nho);
+void vec_folds(const Dev& d, const uint32_t* slots, uint32_t count, int p, cudaStream_t s);
 // Chance nodes of one level (no runout terminals), and its chance edges' reach
 // for the players of qmask.
 void vec_chance(const Dev& d, const ChanceItem* items, uint32_t count, int p, cudaStream_t s);

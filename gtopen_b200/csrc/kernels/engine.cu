@@ -118,6 +118,8 @@ struct EngineImpl {
     ShowItem* show = nullptr;
     ShowBatch* show_batch = nullptr;
     ShowGroups shows, shows_upper;  // vector kernels: every showdown / those outside river rounds
+    uint32_t nfolds = 0;            // vector kernels: action nodes with a fold child,
+    uint32_t* fold_slots[2] = {nullptr, nullptr};  // per traverser the opponent's reach slot of each
     ChanceItem* chance = nullptr;
     XNode* xnodes[2] = {nullptr, nullptr};
     std::vector<XNode> hx[2];
@@ -455,7 +457,17 @@ struct EngineImpl {
         const bool fork = pr == nullptr && side != nullptr && !vec;
         if (vec) {
             const ShowGroups& sg = use_river() ? shows_upper : shows;
-            if (sg.count) timed(pr, 4, [&] { vec_show(d, sg, p, stream); });
+            if (pr || !side) {
+                if (sg.count) timed(pr, 4, [&] { vec_show(d, sg, p, stream); });
+                timed(pr, 6, [&] { vec_folds(d, fold_slots[p], nfolds, p, stream); });  // counted with the action nodes
+            } else {
+                CK(cudaEventRecord(ev_fork, stream));
+                CK(cudaStreamWaitEvent(side, ev_fork, 0));
+                vec_folds(d, fold_slots[p], nfolds, p, side);
+                CK(cudaEventRecord(ev_join, side));
+                vec_show(d, sg, p, stream);
+                CK(cudaStreamWaitEvent(stream, ev_join, 0));
+            }
         }
         if (fork) {
             CK(cudaEventRecord(ev_fork, stream));
@@ -844,7 +856,26 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     E.show_smem = (size_t)d.scr_elems * sizeof(double);
     if (E.warp) E.warp_smem = (size_t)kWarps * d.nh_pad * sizeof(float);
     if (E.vec) {
-        // node records, packed hand words
+        // node records, packed hand words; folds numbered in record order
+        std::vector<uint32_t> fold_no(P.act.size(), 0), fs[2];
+        for (size_t k = 0; k < P.act.size(); k++) {
+            const ActItem& a = P.act[k];
+            if (!a.nterm) continue;  // in-place terminals: folds only
+            fold_no[k] = (uint32_t)fs[0].size();
+            for (uint32_t c = 0; c < a.na; c++)
+                if (P.crefs[a.cref + c].kind == kChildFold) {
+                    fs[a.actor].push_back(a.oslot);                        // the traverser folds: the opponent's reach here
+                    fs[1 - a.actor].push_back(P.crefs[a.cref + c].rslot);  // the opponent does: its reach at the fold
+                }
+        }
+        E.nfolds = (uint32_t)fs[0].size();
+        for (int q = 0; q < 2; q++) {
+            E.fold_slots[q] = dupload(fs[q], O, &B);
+            size_t fsm;
+            const void* fn = fold_kernel(&fsm, P.nh[q]);
+            set_smem(fn, fsm);
+        }
+        d.folds = (const FoldSum*)dalloc((size_t)E.nfolds * fold_sum_bytes(), O, &B);
         auto records = [&](auto KA) {
             constexpr int K = KA();
             PodVec<SNodeT<K>> sn(P.act.size());
@@ -871,6 +902,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
                         if (r.kind == kChildFold) {
                             const TermInfo& t = P.terms[r.term];
                             x.fk = c;
+                            x.cs[c] = fold_no[k];
                             x.folder = t.aux;
                             x.twin = t.twin;
                             x.tlose = t.tlose;
