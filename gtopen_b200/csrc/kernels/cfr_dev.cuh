@@ -218,6 +218,13 @@ struct alignas(16) SNodeT {
     uint32_t folder;           // the folding player of the fold child
     float twin, tlose;         // fold payoffs
 };
+// Programmatic dependent launch: a kernel lets the next one on its stream
+// take free SMs as soon as all its own CTAs run, and waits for the one before
+// it to finish before it touches anything that one may write.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 // One fold's opponent reach vector, summarised (game.rs:478-485) with exact
 // sums: per card, in total, and the grid scale they are on.
 struct alignas(16) FoldSum {

@@ -280,6 +280,7 @@ __global__ void __launch_bounds__(NT) kv_show(Dev d, const ShowItem* items, cons
         uint4* im = (uint4*)(sm + SL.o_img);
         for (int k = tid; k < il / 8; k += NT) im[k] = src[k];
     }
+    pdl_enter();  // items, images and ranks are constant; reach is not
     uint32_t mx = stage_interleaved<G, NT>(pick(d.reach, o) + (size_t)it.rs[o] * pick(d.rstr, o), it.cslot != kNoSlot, nho,
                                            nho_pad, (float*)(sm + SL.o_r));
 #pragma unroll
@@ -322,6 +323,7 @@ __global__ void __launch_bounds__(kFoldThreads) kv_folds(Dev d, const uint32_t* 
     const uint32_t f0 = blockIdx.x * G, fg = f0 + (uint32_t)g;
     if (tid < G) s_mx[tid] = 0u;
     const float* src = pick(d.reach, o) + (size_t)(fg < count ? slots[fg] : 0u) * pick(d.rstr, o);
+    pdl_enter();
     uint32_t mx = stage_interleaved<G, kFoldThreads>(src, fg < count, nho, nho_pad, (float*)sm);
 #pragma unroll
     for (int x = G; x < 32; x <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, x));
@@ -430,6 +432,7 @@ __global__ void __launch_bounds__(kChanceThreads) kv_chance(Dev d, const ChanceI
     const ChanceItem c = items[nd];
     for (uint32_t t = threadIdx.x; t < 52 + kChanceBatch; t += kChanceThreads)
         s_c[t] = t < c.cc_count ? d.cards[c.cc_start + t] : CardEntry{0xFFu, 0, 0, 0};
+    pdl_enter();
     __syncthreads();
     const int nh = pick(d.nh, p), i = (int)((blockIdx.x - nd * chunks) * kChanceThreads + threadIdx.x);
     if (i >= nh) return;
@@ -460,6 +463,7 @@ __global__ void __launch_bounds__(256) kv_edges(Dev d, const EdgeItem* items, ui
     const uint32_t e = (uint32_t)(g / quads), k = (uint32_t)(g - (uint64_t)e * quads);
     if (e >= count) return;
     const uint32_t card = items[e].card;
+    pdl_enter();
     const size_t str = (size_t)pick(d.rstr, q);
     float* base = pick(d.reach, q);
     float4 v = ((const float4*)(base + (size_t)items[e].prs[q] * str))[k];
@@ -524,8 +528,8 @@ void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s) {
     const int o = 1 - p;
     const size_t smem = show_group_smem(sg.shape[o], sg.max_sorted[o], d.nh[o]);
     with_show(sg.shape[o], [&](auto G, auto NT, auto K) {
-        kv_show<G(), NT(), K()><<<sg.count, NT(), smem, s>>>(d, sg.items, (const uint16_t*)sg.img[o],
-                                                             (const HandRank*)sg.ranks[p], p, sg.max_sorted[o]);
+        pdl_launch(kv_show<G(), NT(), K()>, sg.count, NT(), smem, s, d, sg.items, (const uint16_t*)sg.img[o],
+                   (const HandRank*)sg.ranks[p], p, sg.max_sorted[o]);
     });
 }
 size_t fold_sum_bytes() { return sizeof(FoldSum); }
@@ -539,13 +543,13 @@ void vec_folds(const Dev& d, const uint32_t* slots, uint32_t count, int p, cudaS
     const int nho = d.nh[1 - p], G = fold_group(nho);
     const unsigned grid = (count + G - 1) / G, smem = (unsigned)((nho + 3) & ~3) * G * 4;
     FoldSum* out = const_cast<FoldSum*>(d.folds);
-    if (G == 8) kv_folds<8><<<grid, kFoldThreads, smem, s>>>(d, slots, count, p, out);
-    else kv_folds<32><<<grid, kFoldThreads, smem, s>>>(d, slots, count, p, out);
+    if (G == 8) pdl_launch(kv_folds<8>, grid, kFoldThreads, smem, s, d, slots, count, p, out);
+    else pdl_launch(kv_folds<32>, grid, kFoldThreads, smem, s, d, slots, count, p, out);
 }
 void vec_chance(const Dev& d, const ChanceItem* items, uint32_t count, int p, cudaStream_t s) {
     if (!count) return;
     const uint32_t chunks = (uint32_t)((d.nh[p] + kChanceThreads - 1) / kChanceThreads);
-    kv_chance<<<count * chunks, kChanceThreads, 0, s>>>(d, items, p, chunks);
+    pdl_launch(kv_chance, count * chunks, kChanceThreads, 0, s, d, items, p, chunks);
 }
 void vec_edges(const Dev& d, const EdgeItem* items, uint32_t count, int qmask, cudaStream_t s) {
     if (!count) return;
@@ -553,7 +557,7 @@ void vec_edges(const Dev& d, const EdgeItem* items, uint32_t count, int qmask, c
         if (!(qmask >> q & 1)) continue;
         const uint32_t quads = (uint32_t)(d.rstr[q] / 4);
         const uint64_t n = (uint64_t)count * quads;
-        kv_edges<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, items, count, q, quads);
+        pdl_launch(kv_edges, (unsigned)((n + 255) / 256), 256, 0, s, d, items, count, q, quads);
     }
 }
 

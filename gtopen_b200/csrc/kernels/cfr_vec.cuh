@@ -265,12 +265,14 @@ __global__ void __launch_bounds__(128) kv_down(Dev d, Arenas ar, const SNodeT<KA
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
     if (n >= count) return;
     const SNodeT<KA>& it = nodes[n];
+    const uint32_t na = it.na;  // the record: constant, on its way while this waits
+    pdl_enter();
     const int i0 = (int)((w - n * wn) * 32 + (threadIdx.x & 31)) * V;
 #define V_CASE(NA)                                                                    \
     case NA:                                                                          \
         if (NA <= KA) v_down_node<FMT, SRC, NA <= KA ? NA : 1, V>(d, ar, it, i0);     \
         break;
-    switch (it.na) {  // uniform per warp: one body per action count
+    switch (na) {  // uniform per warp: one body per action count
         V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
     }
 }
@@ -517,13 +519,15 @@ __global__ void __launch_bounds__(128) kv_up_opp(Dev d, const SNodeT<KA>* nodes,
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
     if (n >= count) return;
     const SNodeT<KA>& it = nodes[n];
+    const uint32_t na = it.na;  // the record: constant, on its way while this waits
+    pdl_enter();
     const int i0 = (int)((w - n * wn) * 32 + (threadIdx.x & 31)) * V;
 #undef V_CASE
 #define V_CASE(NA)                                                    \
     case NA:                                                          \
         if (NA <= KA) v_opp_node<NA <= KA ? NA : 1, V>(d, it, p, i0); \
         break;
-    switch (it.na) {
+    switch (na) {
         V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
     }
 }
@@ -534,13 +538,15 @@ __global__ void __launch_bounds__(128) kv_up_mine(Dev d, Arenas ar, const SNodeT
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
     if (n >= count) return;
     const SNodeT<KA>& it = nodes[n];
+    const uint32_t na = it.na;  // the record: constant, on its way while this waits
+    pdl_enter();
     const int i0 = (int)((w - n * wn) * 32 + (threadIdx.x & 31)) * V;
 #undef V_CASE
 #define V_CASE(NA)                                                                                               \
     case NA:                                                                                                     \
         if (NA <= KA) v_mine_node<FMT, EVAL, PRED, true, NA <= KA ? NA : 1, V>(d, ar, it, p, mode, i0, Group{}); \
         break;
-    switch (it.na) {
+    switch (na) {
         V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
     }
 }
@@ -552,13 +558,15 @@ __global__ void __launch_bounds__(WARP ? 128 : (1326 + 32 * V - 1) / (32 * V) * 
     const uint32_t n = WARP ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
     if (n >= count) return;
     const SNodeT<KA>& it = nodes[n];
+    const uint32_t na = it.na;  // the record: constant, on its way while this waits
+    pdl_enter();
     const Group g{(int)(WARP ? threadIdx.x & 31 : threadIdx.x), (int)(blockDim.x >> 5), red};
 #undef V_CASE
 #define V_CASE(NA)                                                                                        \
     case NA:                                                                                              \
         if (NA <= KA) v_mine_node<FMT, 0, PRED, WARP, NA <= KA ? NA : 1, V>(d, ar, it, p, 0, g.t * V, g); \
         break;
-    switch (it.na) {
+    switch (na) {
         V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
     }
 }
@@ -594,9 +602,9 @@ void down_t(const Dev& d, const Arenas& ar, const VecNodes& n, int nh, int mode,
     const auto* nodes = (const SNodeT<KA>*)n.nodes;
     with_lanes(nh, n.count, [&](auto V, uint32_t wn, unsigned grid) {
         constexpr int v = V();
-        if (mode) kv_down<FMT, kVAverage, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn);
-        else if (ar.pred[0]) kv_down<FMT, kVPredicted, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn);
-        else kv_down<FMT, kVRegret, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn);
+        if (mode) pdl_launch(kv_down<FMT, kVAverage, v, KA>, grid, 128, 0, s, d, ar, nodes, n.count, wn);
+        else if (ar.pred[0]) pdl_launch(kv_down<FMT, kVPredicted, v, KA>, grid, 128, 0, s, d, ar, nodes, n.count, wn);
+        else pdl_launch(kv_down<FMT, kVRegret, v, KA>, grid, 128, 0, s, d, ar, nodes, n.count, wn);
     });
 }
 template <int FMT, int KA>
@@ -607,10 +615,10 @@ void up_mine_t(const Dev& d, const Arenas& ar, const VecNodes& n, int p, int eva
         with_lanes(nh, n.count, [&](auto V, uint32_t wn, unsigned grid) {
             constexpr int v = V();
             if (eval >= 0) {
-                kv_up_mine<FMT, 1, false, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn, p, eval);
+                pdl_launch(kv_up_mine<FMT, 1, false, v, KA>, grid, 128, 0, s, d, ar, nodes, n.count, wn, p, eval);
             } else if constexpr (FMT == kDevF32) {
-                if (ar.pred[0]) kv_up_mine<FMT, 0, true, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn, p, 0);
-                else kv_up_mine<FMT, 0, false, v, KA><<<grid, 128, 0, s>>>(d, ar, nodes, n.count, wn, p, 0);
+                if (ar.pred[0]) pdl_launch(kv_up_mine<FMT, 0, true, v, KA>, grid, 128, 0, s, d, ar, nodes, n.count, wn, p, 0);
+                else pdl_launch(kv_up_mine<FMT, 0, false, v, KA>, grid, 128, 0, s, d, ar, nodes, n.count, wn, p, 0);
             }
         });
         return;
@@ -621,8 +629,8 @@ void up_mine_t(const Dev& d, const Arenas& ar, const VecNodes& n, int p, int eva
             constexpr int v = V();
             const unsigned grid = W ? (n.count + 3) / 4 : n.count;
             const unsigned block = W ? 128u : (unsigned)((nh + 32 * v - 1) / (32 * v)) * 32u;
-            if (ar.pred[0]) kv_up_quant<FMT, true, W, v, KA><<<grid, block, 0, s>>>(d, ar, nodes, n.count, p);
-            else kv_up_quant<FMT, false, W, v, KA><<<grid, block, 0, s>>>(d, ar, nodes, n.count, p);
+            if (ar.pred[0]) pdl_launch(kv_up_quant<FMT, true, W, v, KA>, grid, block, 0, s, d, ar, nodes, n.count, p);
+            else pdl_launch(kv_up_quant<FMT, false, W, v, KA>, grid, block, 0, s, d, ar, nodes, n.count, p);
         };
         // small launches: a CTA per node with fewer hands a thread
         const bool small = (uint64_t)n.count * (uint32_t)((nh + 127) / 128) <= kVFillWarps / 2;
@@ -637,7 +645,7 @@ template <int KA>
 void up_opp_t(const Dev& d, const VecNodes& n, int p, cudaStream_t s) {
     with_lanes(d.nh[p], n.count, [&](auto V, uint32_t wn, unsigned grid) {
         constexpr int v = V();
-        kv_up_opp<v, KA><<<grid, 128, 0, s>>>(d, (const SNodeT<KA>*)n.nodes, n.count, wn, p);
+        pdl_launch(kv_up_opp<v, KA>, grid, 128, 0, s, d, (const SNodeT<KA>*)n.nodes, n.count, wn, p);
     });
 }
 }  // namespace

@@ -6,6 +6,22 @@
 
 namespace gtob {
 
+// A launch of a kernel that starts with pdl_enter().
+template <class... P, class... A>
+void pdl_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // an error stays for the caller's cudaGetLastError
+}
+
 // Action nodes of one level and one actor, given as SNodeT<4> records or
 // (wide) SNodeT<8> records.
 struct VecNodes {
