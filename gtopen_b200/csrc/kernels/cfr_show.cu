@@ -308,13 +308,17 @@ __global__ void __launch_bounds__(NT) kv_show(Dev d, const ShowItem* items, cons
 // barrier at all.  470 v 647 hands, 85,413 folds: 0.13 ms a sweep (issue 74%
 // of peak, the conversions 52%).  One iteration before -> after: that flop,
 // 16-bit, 3.9 -> 3.7 ms; turn f32 0.364 -> 0.291; river f32 0.072 -> 0.058.
-constexpr int kFoldThreads = 256;
+// threads: 52 card lists x 4 lanes (8 folds) x 2 halves of a list, and 26 x 16
+// lanes (32 folds), are 416 -- every thread has a list; a launch that fills
+// the device is faster without the halves' extra steps
+template <int G, int PARTS>
+constexpr int fold_threads() { return G == 8 && PARTS == 1 ? 256 : 416; }
 // folds per CTA: short lists leave a CTA of 8 with more set-up than sums
 inline int fold_group(int nho) { return nho <= 128 ? 32 : 8; }
-template <int G>
-__global__ void __launch_bounds__(kFoldThreads) kv_folds(Dev d, const uint32_t* slots, uint32_t count, int p,
+template <int G, int PARTS>
+__global__ void __launch_bounds__(fold_threads<G, PARTS>()) kv_folds(Dev d, const uint32_t* slots, uint32_t count, int p,
                                                          FoldSum* out) {
-    constexpr int L = G / 2, NC = kFoldThreads / L;
+    constexpr int L = G / 2, NT = fold_threads<G, PARTS>(), NC = NT / L / PARTS;
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ uint32_t s_mx[G];
     __shared__ longlong2 s_S[52 * L];
@@ -324,13 +328,13 @@ __global__ void __launch_bounds__(kFoldThreads) kv_folds(Dev d, const uint32_t* 
     if (tid < G) s_mx[tid] = 0u;
     const float* src = pick(d.reach, o) + (size_t)(fg < count ? slots[fg] : 0u) * pick(d.rstr, o);
     pdl_enter();
-    uint32_t mx = stage_interleaved<G, kFoldThreads>(src, fg < count, nho, nho_pad, (float*)sm);
+    uint32_t mx = stage_interleaved<G, NT>(src, fg < count, nho, nho_pad, (float*)sm);
 #pragma unroll
     for (int x = G; x < 32; x <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, x));
     __syncthreads();
     if ((tid & 31) < G) atomicMax(&s_mx[g], mx);
     __syncthreads();
-    const int l = tid & (L - 1), c_ = tid / L;
+    const int l = tid & (L - 1), part = tid / L % PARTS, c_ = tid / (L * PARTS);
     const Grid ga = make_grid(__uint_as_float(s_mx[2 * l])), gb = make_grid(__uint_as_float(s_mx[2 * l + 1]));
     const uint32_t fa = f0 + 2 * (uint32_t)l;
     const bool onA = fa < count, onB = fa + 1 < count;
@@ -341,19 +345,25 @@ __global__ void __launch_bounds__(kFoldThreads) kv_folds(Dev d, const uint32_t* 
         longlong2 a = make_longlong2(0, 0);
         const bool big = ga.S > 126 || gb.S > 126;
 #pragma unroll 4
-        for (uint32_t k = b; k < e; k++) {
+        for (uint32_t k = b + part; k < e; k += PARTS) {
             const float2 x = r2[(int)idx[k] * L];
             a.x += big ? grid_q<true>(ga, x.x) : grid_q<false>(ga, x.x);
             a.y += big ? grid_q<true>(gb, x.y) : grid_q<false>(gb, x.y);
         }
-        s_S[c * L + l] = a;
-        if (onA) out[fa].S[c] = a.x;
-        if (onB) out[fa + 1].S[c] = a.y;
+        if (PARTS == 2) {  // the other half's lane (every warp is whole here: one round)
+            a.x += __shfl_xor_sync(0xffffffffu, a.x, L);
+            a.y += __shfl_xor_sync(0xffffffffu, a.y, L);
+        }
+        if (part == 0) {
+            s_S[c * L + l] = a;
+            if (onA) out[fa].S[c] = a.x;
+            if (onB) out[fa + 1].S[c] = a.y;
+        }
     }
     __syncthreads();
     if (tid < 32) {  // every hand holds two cards: the total is half the card sums' sum
         longlong2 t = make_longlong2(0, 0);
-        for (int k = c_; k < 52; k += 32 / L) {
+        for (int k = tid / L; k < 52; k += 32 / L) {
             t.x += s_S[k * L + l].x;
             t.y += s_S[k * L + l].y;
         }
@@ -422,38 +432,43 @@ __global__ void k_show_images(Dev d, int o, int msort, int K, uint16_t* out) {
 // ------------------------------------------------------------ chance nodes
 // Chance node without runout terminals (cfr.rs:637-663): per hand the sum of
 // its representatives' children in card order, times 1 / divisor.  One hand
-// per thread, `chunks` CTAs per node; the children's values are loaded sixteen
-// cards at a time and added in order (a skipped card adds +0, which changes
+// per lane, `chunks` CTAs per node; four threads load a hand's children, all 52
+// cards' loads in flight, and one adds them in card order (a skipped card adds +0, which changes
 // no bits of a sum that starts at +0).
-constexpr int kChanceThreads = 64, kChanceBatch = 16;
-__global__ void __launch_bounds__(kChanceThreads) kv_chance(Dev d, const ChanceItem* items, int p, uint32_t chunks) {
-    __shared__ CardEntry s_c[52 + kChanceBatch];
+constexpr int kChanceHands = 64, kChanceParts = 4;
+__global__ void __launch_bounds__(kChanceHands* kChanceParts) kv_chance(Dev d, const ChanceItem* items, int p,
+                                                                        uint32_t chunks) {
+    constexpr int NT = kChanceHands * kChanceParts, N = 52 / kChanceParts;
+    __shared__ CardEntry s_c[52];
+    __shared__ float s_v[52][kChanceHands];
     const uint32_t nd = blockIdx.x / chunks;
     const ChanceItem c = items[nd];
-    for (uint32_t t = threadIdx.x; t < 52 + kChanceBatch; t += kChanceThreads)
-        s_c[t] = t < c.cc_count ? d.cards[c.cc_start + t] : CardEntry{0xFFu, 0, 0, 0};
+    if (threadIdx.x < 52)
+        s_c[threadIdx.x] = threadIdx.x < c.cc_count ? d.cards[c.cc_start + threadIdx.x] : CardEntry{0xFFu, 0, 0, 0};
+    const int nh = pick(d.nh, p), h = (int)threadIdx.x % kChanceHands, part = (int)threadIdx.x / kChanceHands;
+    const int i = (int)(blockIdx.x - nd * chunks) * kChanceHands + h;
+    const uint64_t hm = i < nh ? pick(d.mask, p)[i] : ~0ull;
+    const uint16_t* hp = pick(d.hperm, p);
     pdl_enter();
     __syncthreads();
-    const int nh = pick(d.nh, p), i = (int)((blockIdx.x - nd * chunks) * kChanceThreads + threadIdx.x);
-    if (i >= nh) return;
-    const uint64_t hm = pick(d.mask, p)[i];
-    const uint16_t* hp = pick(d.hperm, p);
-    float acc = 0.0f;
-    for (uint32_t t0 = 0; t0 < c.cc_count; t0 += kChanceBatch) {
-        float v[kChanceBatch];
+    float v[N];
 #pragma unroll
-        for (uint32_t j = 0; j < kChanceBatch; j++) {
-            const CardEntry e = s_c[t0 + j];
-            const uint32_t card = e.card & 0xFF;
-            v[j] = 0.0f;
-            if (card < 52u && !(hm >> card & 1ull)) {
-                const int src = e.perm ? (int)hp[(size_t)e.perm * nh + i] : i;
-                v[j] = d.cfv[(size_t)e.child_cslot * d.nh_max + src];
-            }
+    for (int j = 0; j < N; j++) {
+        const CardEntry e = s_c[part * N + j];
+        const uint32_t card = e.card & 0xFF;
+        v[j] = 0.0f;
+        if (card < 52u && !(hm >> card & 1ull)) {
+            const int src = e.perm ? (int)hp[(size_t)e.perm * nh + i] : i;
+            v[j] = d.cfv[(size_t)e.child_cslot * d.nh_max + src];
         }
-#pragma unroll
-        for (uint32_t j = 0; j < kChanceBatch; j++) acc += v[j];
     }
+#pragma unroll
+    for (int j = 0; j < N; j++) s_v[part * N + j][h] = v[j];
+    __syncthreads();
+    if (part != 0 || i >= nh) return;
+    float acc = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 52; t++) acc += s_v[t][h];
     d.cfv[(size_t)c.cslot * d.nh_max + i] = acc * c.inv;
 }
 // Chance edges of player q: the parent's reach with the holders of the card
@@ -533,23 +548,25 @@ void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s) {
     });
 }
 size_t fold_sum_bytes() { return sizeof(FoldSum); }
-const void* fold_kernel(size_t* smem, int nho) {
+void fold_kernels(int nho, const void* (&fn)[2], size_t* smem) {
     const int G = fold_group(nho);
     *smem = (size_t)((nho + 3) & ~3) * G * 4;
-    return G == 8 ? (const void*)kv_folds<8> : (const void*)kv_folds<32>;
+    fn[0] = G == 8 ? (const void*)kv_folds<8, 1> : (const void*)kv_folds<32, 1>;
+    fn[1] = G == 8 ? (const void*)kv_folds<8, 2> : fn[0];
 }
 void vec_folds(const Dev& d, const uint32_t* slots, uint32_t count, int p, cudaStream_t s) {
     if (!count) return;
     const int nho = d.nh[1 - p], G = fold_group(nho);
     const unsigned grid = (count + G - 1) / G, smem = (unsigned)((nho + 3) & ~3) * G * 4;
     FoldSum* out = const_cast<FoldSum*>(d.folds);
-    if (G == 8) pdl_launch(kv_folds<8>, grid, kFoldThreads, smem, s, d, slots, count, p, out);
-    else pdl_launch(kv_folds<32>, grid, kFoldThreads, smem, s, d, slots, count, p, out);
+    if (G == 32) pdl_launch(kv_folds<32, 1>, grid, fold_threads<32, 1>(), smem, s, d, slots, count, p, out);
+    else if (grid <= 148 * 3) pdl_launch(kv_folds<8, 2>, grid, fold_threads<8, 2>(), smem, s, d, slots, count, p, out);
+    else pdl_launch(kv_folds<8, 1>, grid, fold_threads<8, 1>(), smem, s, d, slots, count, p, out);
 }
 void vec_chance(const Dev& d, const ChanceItem* items, uint32_t count, int p, cudaStream_t s) {
     if (!count) return;
-    const uint32_t chunks = (uint32_t)((d.nh[p] + kChanceThreads - 1) / kChanceThreads);
-    pdl_launch(kv_chance, count * chunks, kChanceThreads, 0, s, d, items, p, chunks);
+    const uint32_t chunks = (uint32_t)((d.nh[p] + kChanceHands - 1) / kChanceHands);
+    pdl_launch(kv_chance, count * chunks, kChanceHands * kChanceParts, 0, s, d, items, p, chunks);
 }
 void vec_edges(const Dev& d, const EdgeItem* items, uint32_t count, int qmask, cudaStream_t s) {
     if (!count) return;

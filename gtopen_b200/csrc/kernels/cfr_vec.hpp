@@ -64,7 +64,7 @@ void vec_show(const Dev& d, const ShowGroups& sg, int p, cudaStream_t s);
 // A sweep's fold summaries into d.folds: fold k's opponent vector is reach
 // slot slots[k].
 size_t fold_sum_bytes();
-const void* fold_kernel(size_t* smem, int nho);
+void fold_kernels(int nho, const void* (&fn)[2], size_t* smem);
 void vec_folds(const Dev& d, const uint32_t* slots, uint32_t count, int p, cudaStream_t s);
 // Chance nodes of one level (no runout terminals), and its chance edges' reach
 // for the players of qmask.

@@ -935,8 +935,9 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
         for (int q = 0; q < 2; q++) {
             E.fold_slots[q] = dupload(fs[q], O, &B);
             size_t fsm;
-            const void* fn = fold_kernel(&fsm, P.nh[q]);
-            set_smem(fn, fsm);
+            const void* fn[2];
+            fold_kernels(P.nh[q], fn, &fsm);
+            for (const void* f : fn) set_smem(f, fsm);
         }
         d.folds = (const FoldSum*)dalloc((size_t)E.nfolds * fold_sum_bytes(), O, &B);
         auto records = [&](auto KA) {
