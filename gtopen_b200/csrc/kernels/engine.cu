@@ -42,6 +42,7 @@
 #include "cfr_batch.cuh"
 #include "cfr_vec.hpp"
 #include "engine.hpp"
+#include "../host/hostcopy.hpp"
 
 namespace gtob {
 
@@ -153,7 +154,8 @@ struct EngineImpl {
     size_t chance_smem = 0;  // runout chance dynamic smem
     cudaGraphExec_t g_iter = nullptr;
     cudaGraphExec_t g_eval[2] = {nullptr, nullptr};
-    double* h_dot = nullptr;  // pinned
+    double* h_dot = nullptr;       // pinned, with the read-back chunks behind it
+    unsigned char* pin = nullptr;  // 2 * kPinChunk
 
     // Two pinned chunks for large device -> pageable host copies (allocated
     // on first use): the DMA of one chunk overlaps the spread copy of the
@@ -163,9 +165,8 @@ struct EngineImpl {
     unsigned char* d2h_pin[2] = {nullptr, nullptr};
     cudaEvent_t d2h_ev[2] = {nullptr, nullptr};
     void d2h_large(void* dst, const void* src, size_t bytes) {
-        if (bytes < 2 * kD2HChunk) {
-            CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
-            CK(cudaStreamSynchronize(stream));
+        if (bytes < 2 * kD2HChunk) {  // small chunks, pinned with the engine
+            copy_to_host(dst, src, bytes, stream, pin);
             return;
         }
         for (int b = 0; b < 2; b++)
@@ -901,19 +902,20 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
         d.node_id[q] = dupload(P.anode_id[q], O, &B);
     }
     d.cards = dupload(P.cards, O, &B);
-    d.crefs = dupload(P.crefs, O, &B);
-    d.terms = dupload(P.terms, O, &B);
+    if (!E.vec) {  // the vector kernels' node records hold all of it
+        d.crefs = dupload(P.crefs, O, &B);
+        d.terms = dupload(P.terms, O, &B);
+    }
     d.cfv = (float*)dalloc(P.n_cslots * (size_t)d.nh_max * sizeof(float), O, &B);
     d.disc = (float*)dalloc(4 * sizeof(float), O, &B);
     d.iter = (unsigned*)dalloc(sizeof(unsigned), O, &B);
     d.dot = (double*)dalloc(4 * sizeof(double), O, &B);
     d.err = (unsigned*)dalloc(sizeof(unsigned), O, &B);
     CK(cudaMemcpy(d.iter, &E.iteration, sizeof(unsigned), cudaMemcpyHostToDevice));
-    E.act = dupload(P.act, O, &B);
+    if (!E.vec) E.act = dupload(P.act, O, &B);
     E.edge = dupload(P.edge, O, &B);
     E.fold = dupload(P.fold, O, &B);
-    E.show = dupload(P.show, O, &B);
-    E.show_batch = dupload(P.show_batch, O, &B);
+    if (!E.vec) E.show = dupload(P.show, O, &B);
     E.chance = dupload(P.chance, O, &B);
     const size_t tsz = E.term64 ? sizeof(double) : sizeof(float);
     E.show_smem = (size_t)d.scr_elems * sizeof(double);
@@ -1035,7 +1037,10 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     }
     E.staging_len = std::max<uint64_t>(std::max(sp.tree.data_size[0], sp.tree.data_size[1]), 1);
     E.staging = (float*)dalloc(E.staging_len * sizeof(float), O, &B);
-    CK(cudaMallocHost(&E.h_dot, 4 * sizeof(double)));
+    // read-back chunks only where an arena is worth them (pinning takes a few ms)
+    const bool big = E.staging_len * sizeof(float) >= 2 * kPinChunk;
+    CK(cudaMallocHost(&E.h_dot, 4096 + (big ? 2 * kPinChunk : 0)));
+    if (big) E.pin = (unsigned char*)E.h_dot + 4096;
 
     // upload arenas: quants directly when host and device are both 16-bit, else via f32 (+ encode);
     // nothing to upload while the host arenas are still all zero (so are the device's)
@@ -1827,7 +1832,11 @@ struct BatchImpl {
         smem = 16;
         std::vector<const Plan*> plans;
         for (size_t s = 0; s < E.size(); s++) {
-            const EngineImpl& X = *E[s];
+            EngineImpl& X = *E[s];
+            if (!X.show) {  // the level-ordered showdowns: the batched kernel's only
+                X.show = dupload(X.plan.show, X.owned, &X.bytes);
+                X.show_batch = dupload(X.plan.show_batch, X.owned, &X.bytes);
+            }
             BSpot& b = hs[s];
             std::memset(&b, 0, sizeof(b));
             b.d = X.d;

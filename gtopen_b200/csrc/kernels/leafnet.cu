@@ -383,10 +383,10 @@ CUtensorMap tile_map(const void* base, uint64_t inner, uint64_t rows, uint32_t b
     return m;
 }
 template <class T>
-T* dnew(size_t n) {
+T* dnew(size_t n, bool zeroed = true) {
     void* p = nullptr;
     LCK(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
-    LCK(cudaMemset(p, 0, std::max<size_t>(n, 1) * sizeof(T)));
+    if (zeroed) LCK(cudaMemset(p, 0, std::max<size_t>(n, 1) * sizeof(T)));
     return (T*)p;
 }
 int pad128(int x) { return (x + 127) / 128 * 128; }
@@ -692,7 +692,7 @@ namespace {
 template <class T>
 struct DevBuf {
     T* p = nullptr;
-    explicit DevBuf(size_t n) : p(dnew<T>(n)) {}
+    explicit DevBuf(size_t n, bool zeroed = true) : p(dnew<T>(n, zeroed)) {}
     ~DevBuf() { cudaFree(p); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -701,7 +701,9 @@ struct DevBuf {
 struct DevTable {
     DevBuf<float> buf;
     float* p;
-    DevTable(const float* h, size_t n) : buf(n), p(buf.p) { LCK(cudaMemcpy(p, h, n * 4, cudaMemcpyHostToDevice)); }
+    DevTable(const float* h, size_t n) : buf(n, false), p(buf.p) {
+        LCK(cudaMemcpy(p, h, n * 4, cudaMemcpyHostToDevice));
+    }
 };
 }  // namespace
 
