@@ -41,14 +41,15 @@ namespace gtob {
 
 namespace {
 
-constexpr int kBM = 128, kBK = 64, kStages = 4;
+constexpr int kBM = 128, kBK = 64;
 constexpr int kGemmThreads = 128;
 constexpr uint32_t kTileABytes = kBM * kBK * 2;
 constexpr unsigned long long kNetWaitNs = 2000000000ull;
 constexpr unsigned kErrGemmWait = 16u;
-// A 128 x BN output tile (BN = 128 or 256: TMEM columns, B rows per stage).
+// A 128 x BN output tile (BN TMEM columns, B rows per stage).
 template <int BN>
 struct TileCfg {
+    static constexpr int kStages = BN >= 128 ? 4 : 5;
     static constexpr uint32_t kTileB = BN * kBK * 2;
     static constexpr uint32_t kStage = kTileABytes + kTileB;
     static constexpr size_t kSmem = (size_t)kStages * kStage + 1024;  // + room to align the ring to 1 KiB
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
               unsigned* err) {
     extern __shared__ uint8_t dsm[];
     uint8_t* ring = dsm + ((1024u - (su32(dsm) & 1023u)) & 1023u);  // 1 KiB aligned: the swizzle atoms
+    constexpr int kStages = TileCfg<BN>::kStages;
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t tbase;
     __shared__ int aborted, issued;
@@ -289,21 +291,22 @@ __global__ void k_transpose(const __nv_bfloat16* __restrict__ in, int R, int C, 
     __syncthreads();
     for (int j = threadIdx.y; j < 32; j += blockDim.y) out[(size_t)(c0 + j) * R + r0 + threadIdx.x] = t[threadIdx.x][j];
 }
-// rows of a row-major f32 table (row idx[i] of width w) into padded buffers:
-// bf16 (x) or f32 (y); padding rows and columns zero
-__global__ void k_gather_rows_bf16(const float* __restrict__ src, const int* __restrict__ idx, int n, int w, int wp,
-                                   __nv_bfloat16* __restrict__ dst) {
-    const int r = blockIdx.x;
-    for (int c = threadIdx.x; c < wp; c += blockDim.x) {
-        const float v = r < n && c < w ? src[(size_t)idx[r] * w + c] : 0.0f;
-        dst[(size_t)r * wp + c] = __float2bfloat16_rn(v);
+// A batch's rows idx[0..n) of the f32 tables into the padded buffers: inputs
+// as bf16, targets and masks as f32; padding rows and columns zero.  tt == null:
+// inputs only.  One launch, a row split over gridDim.y blocks.
+__global__ void k_gather_rows(const float* __restrict__ x, const float* __restrict__ t, const float* __restrict__ m,
+                              const int* __restrict__ idx, int n, int din, int din_p, int dout, int dout_p,
+                              __nv_bfloat16* __restrict__ xx, float* __restrict__ tt, float* __restrict__ mm) {
+    const int r = blockIdx.x, step = blockDim.x * gridDim.y, c0 = blockIdx.y * blockDim.x + threadIdx.x;
+    const size_t row = r < n ? (size_t)idx[r] : 0;
+    for (int c = c0; c < din_p; c += step)
+        xx[(size_t)r * din_p + c] = __float2bfloat16_rn(r < n && c < din ? x[row * din + c] : 0.0f);
+    if (!tt) return;
+    for (int c = c0; c < dout_p; c += step) {
+        const bool in = r < n && c < dout;
+        tt[(size_t)r * dout_p + c] = in ? t[row * dout + c] : 0.0f;
+        mm[(size_t)r * dout_p + c] = in ? m[row * dout + c] : 0.0f;
     }
-}
-__global__ void k_gather_rows_f32(const float* __restrict__ src, const int* __restrict__ idx, int n, int w, int wp,
-                                  float* __restrict__ dst) {
-    const int r = blockIdx.x;
-    for (int c = threadIdx.x; c < wp; c += blockDim.x)
-        dst[(size_t)r * wp + c] = r < n && c < w ? src[(size_t)idx[r] * w + c] : 0.0f;
 }
 // masked squared error, averaged over n * w entries: dy = d loss / d y (f32
 // and bf16), loss accumulated in f64
@@ -328,29 +331,88 @@ __global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t,
         atomicAdd(loss, s * (double)inv);
     }
 }
-// out[c] = sum over rows of g[r * N + c]
-__global__ void k_colsum(const float* __restrict__ g, int rows, int N, float* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
+// out[c] = sum over rows of g[r * N + c], rows added in order: 128 rows of 32
+// columns at a time through shared memory, so that the loads do not wait for
+// the additions (N a multiple of 32).  256 rows: 13 -> 4 us.
+__global__ void __launch_bounds__(256) k_colsum(const float* __restrict__ g, int rows, int N, float* __restrict__ out) {
+    __shared__ float t[128][33];
+    const int c = threadIdx.x & 31, w = threadIdx.x >> 5, c0 = blockIdx.x * 32;
     float s = 0.0f;
-    for (int r = 0; r < rows; r++) s += g[(size_t)r * N + c];
-    out[c] = s;
+    for (int r0 = 0; r0 < rows; r0 += 128) {
+        const int n = min(128, rows - r0);
+#pragma unroll 16
+        for (int k = w; k < n; k += 8) t[k][c] = g[(size_t)(r0 + k) * N + c0 + c];
+        __syncthreads();
+        if (w == 0) {
+#pragma unroll 16
+            for (int k = 0; k < n; k++) s += t[k][c];
+        }
+        __syncthreads();
+    }
+    if (w == 0) out[c0 + c] = s;
 }
-// Adam on the f32 masters; refreshes the bf16 copy (mask: padded entries
-// stay zero)
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, const uint8_t* __restrict__ live, size_t n, float lr, float b1, float b2,
-                       float eps, float bc1, float bc2, __nv_bfloat16* __restrict__ wb) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        if (live && !live[i]) continue;
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float step = lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-        w[i] -= step;
-        if (wb) wb[i] = __float2bfloat16_rn(w[i]);
+// One Adam step of every layer in one launch: 32 x 32 tiles of the weights
+// (masters, moments, the bf16 copy and its transpose, which the next step's
+// products read), then the biases; padded weights (live = 0) stay zero.
+// 8.4M parameters: twelve launches, 120 us -> one, bound by HBM.
+struct AdamLayer {
+    float *w, *g, *m, *v, *b, *gb, *mb, *vb;
+    const uint8_t* live;
+    __nv_bfloat16 *wb, *wt;
+    int in_p, out_p, out, tile0, bias0;  // first block of the weights' tiles, of the biases
+};
+constexpr int kAdamLayers = 9;
+struct AdamLayers {
+    AdamLayer l[kAdamLayers];
+    int n;
+};
+__device__ __forceinline__ float adam_one(float& w, float g, float& m, float& v, float lr, float b1, float b2, float eps,
+                                          float bc1, float bc2) {
+    const float mi = b1 * m + (1.0f - b1) * g;
+    const float vi = b2 * v + (1.0f - b2) * g * g;
+    m = mi;
+    v = vi;
+    const float step = lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    w -= step;
+    return w;
+}
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamLayers A, float lr, float b1, float b2,
+                                              float eps, float bc1, float bc2) {
+    __shared__ __nv_bfloat16 t[32][33];
+    const int blk = (int)blockIdx.x, c = threadIdx.x & 31, r0 = threadIdx.x >> 5;
+    for (int k = 0; k < A.n; k++) {
+        const AdamLayer& L = A.l[k];
+        const int tiles = (L.in_p / 32) * (L.out_p / 32);
+        if (blk >= L.tile0 && blk < L.tile0 + tiles) {
+            const int ti = blk - L.tile0, cx = ti % (L.in_p / 32) * 32, ry = ti / (L.in_p / 32) * 32;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int r = r0 + 8 * j;
+                const size_t i = (size_t)(ry + r) * L.in_p + cx + c;
+                __nv_bfloat16 x = __float2bfloat16_rn(0.0f);
+                if (L.live[i]) {
+                    float w = L.w[i], m = L.m[i], v = L.v[i];
+                    x = __float2bfloat16_rn(adam_one(w, L.g[i], m, v, lr, b1, b2, eps, bc1, bc2));
+                    L.w[i] = w;
+                    L.m[i] = m;
+                    L.v[i] = v;
+                    L.wb[i] = x;
+                }
+                t[r][c] = x;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int r = r0 + 8 * j;
+                L.wt[(size_t)(cx + r) * L.out_p + ry + c] = t[c][r];
+            }
+            return;
+        }
+        if (blk >= L.bias0 && blk < L.bias0 + (L.out + 255) / 256) {
+            const int i = (blk - L.bias0) * 256 + (int)threadIdx.x;
+            if (i < L.out) adam_one(L.b[i], L.gb[i], L.mb[i], L.vb[i], lr, b1, b2, eps, bc1, bc2);
+            return;
+        }
     }
 }
 __global__ void k_to_bf16(const float* __restrict__ in, size_t n, __nv_bfloat16* __restrict__ out) {
@@ -389,6 +451,7 @@ T* dnew(size_t n, bool zeroed = true) {
     if (zeroed) LCK(cudaMemset(p, 0, std::max<size_t>(n, 1) * sizeof(T)));
     return (T*)p;
 }
+constexpr int kGatherSplit = 4;
 int pad128(int x) { return (x + 127) / 128 * 128; }
 int grid_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 16); }
 uint64_t xs_next(uint64_t& s) {
@@ -417,14 +480,21 @@ static void launch_gemm(const __nv_bfloat16* A, const __nv_bfloat16* B, int M, i
     LCK(cudaGetLastError());
 }
 
+constexpr int kTilesWanted = 120;
 void gemm_bf16_tn(const __nv_bfloat16* A, const __nv_bfloat16* B, int M, int N, int K, const GemmEpilogue& e,
                   unsigned* err, cudaStream_t s) {
     if (M <= 0 || N <= 0 || K <= 0 || M % kBM || N % 128 || K % kBK)
         throw Error("invalid argument: matrix product shape (M, N multiples of 128, K of 64)");
-    // 128 x 256 tiles where N allows (twice the work per instruction and per
-    // tile, half the tiles), else 128 x 128
-    if (N % 256 == 0) launch_gemm<256>(A, B, M, N, K, e, err, s);
-    else launch_gemm<128>(A, B, M, N, K, e, err, s);
+    // the widest tile that still gives most SMs one: a tile's K loop is a chain
+    // of products whatever its width, so a 256-row batch on eight 128 x 256
+    // tiles left the device idle (256 x 1024 x 1024: 21 us at BN = 256, 16.5
+    // at 128, 12.8 at 64, 11.1 at 32; 4096 x 1024 x 2816 keeps BN = 256)
+    auto tiles = [&](int bn) { return N % bn ? 0 : M / kBM * (N / bn); };
+    int bn = tiles(256) >= kTilesWanted ? 256 : tiles(128) >= kTilesWanted ? 128 : tiles(64) >= kTilesWanted ? 64 : 32;
+    if (bn == 256) launch_gemm<256>(A, B, M, N, K, e, err, s);
+    else if (bn == 128) launch_gemm<128>(A, B, M, N, K, e, err, s);
+    else if (bn == 64) launch_gemm<64>(A, B, M, N, K, e, err, s);
+    else launch_gemm<32>(A, B, M, N, K, e, err, s);
 }
 
 double gemm_time_ms(int m, int n, int k, int reps) {
@@ -488,6 +558,8 @@ LeafNet::LeafNet(const LeafNetDims& d, uint64_t seed) : d_(d) {
     dh_p_ = pad128(d.dh);
     dout_p_ = pad128(d.dout);
     LCK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+    LCK(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
+    LCK(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming));
     err_ = dnew<unsigned>(1);
     loss_ = dnew<double>(1);
     uint64_t s = seed * 0x9E3779B97F4A7C15ull + 0x2545F4914F6CDD1Dull;
@@ -534,6 +606,8 @@ LeafNet::~LeafNet() {
     for (void* p : {(void*)x_, (void*)xt_, (void*)dyb_, (void*)dyt_, (void*)y_, (void*)dy_, (void*)t_, (void*)m_,
                     (void*)loss_, (void*)err_})
         cudaFree(p);
+    if (ev_) cudaEventDestroy(ev_);
+    if (side_) cudaStreamDestroy(side_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -601,11 +675,13 @@ void LeafNet::forward(const __nv_bfloat16* x, int rows_pad, float* y, bool keep,
     launches_++;
 }
 
-double LeafNet::backward(const float* t, const float* mask, int rows_pad, int rows, cudaStream_t s) {
+// The weight gradients (transposes, product, bias column sums) of a layer run
+// on a second stream beside the chain of products that carries the gradient
+// down; s waits for them at the end.
+void LeafNet::backward(const float* t, const float* mask, int rows_pad, int rows, double* loss, cudaStream_t s) {
     const size_t total = (size_t)rows_pad * dout_p_;
-    LCK(cudaMemsetAsync(loss_, 0, sizeof(double), s));
     const float inv = 1.0f / (float)((double)rows * d_.dout);  // the mean over the real rows' entries
-    k_loss<<<grid_for(total), 256, 0, s>>>(y_, t, mask, total, inv, dy_, dyb_, loss_);
+    k_loss<<<grid_for(total), 256, 0, s>>>(y_, t, mask, total, inv, dy_, dyb_, loss);
     launches_++;
     for (int l = d_.nhidden; l >= 0; l--) {
         Layer& L = *L_[l];
@@ -614,13 +690,15 @@ double LeafNet::backward(const float* t, const float* mask, int rows_pad, int ro
         __nv_bfloat16* gt = l == d_.nhidden ? dyt_ : L.dzt;
         const __nv_bfloat16* in = l == 0 ? x_ : L_[l - 1]->h;
         __nv_bfloat16* in_t = l == 0 ? xt_ : L_[l - 1]->ht;
-        k_transpose<<<dim3(L.out_p / 32, rows_pad / 32), dim3(32, 8), 0, s>>>(gb16, rows_pad, L.out_p, gt);
-        k_transpose<<<dim3(L.in_p / 32, rows_pad / 32), dim3(32, 8), 0, s>>>(in, rows_pad, L.in_p, in_t);
+        LCK(cudaEventRecord(ev_, s));
+        LCK(cudaStreamWaitEvent(side_, ev_, 0));
+        k_transpose<<<dim3(L.out_p / 32, rows_pad / 32), dim3(32, 8), 0, side_>>>(gb16, rows_pad, L.out_p, gt);
+        k_transpose<<<dim3(L.in_p / 32, rows_pad / 32), dim3(32, 8), 0, side_>>>(in, rows_pad, L.in_p, in_t);
         GemmEpilogue ew;
         ew.out_f32 = L.gw;
         ew.ld_f32 = L.in_p;
-        gemm_bf16_tn(gt, in_t, L.out_p, L.in_p, rows_pad, ew, err_, s);  // dW = G^T X
-        k_colsum<<<(L.out_p + 127) / 128, 128, 0, s>>>(g32, rows_pad, L.out_p, L.gb);
+        gemm_bf16_tn(gt, in_t, L.out_p, L.in_p, rows_pad, ew, err_, side_);  // dW = G^T X
+        k_colsum<<<L.out_p / 32, 256, 0, side_>>>(g32, rows_pad, L.out_p, L.gb);
         launches_ += 4;
         if (l > 0) {
             Layer& P = *L_[l - 1];
@@ -635,24 +713,28 @@ double LeafNet::backward(const float* t, const float* mask, int rows_pad, int ro
             launches_++;
         }
     }
-    double loss = 0.0;
-    LCK(cudaMemcpyAsync(&loss, loss_, sizeof(double), cudaMemcpyDeviceToHost, s));
-    check(s);
-    return loss;
+    LCK(cudaEventRecord(ev_, side_));
+    LCK(cudaStreamWaitEvent(s, ev_, 0));
+    LCK(cudaGetLastError());
 }
 
 void LeafNet::adam(float lr, int step, cudaStream_t s) {
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float bc1 = (float)(1.0 - std::pow((double)b1, step)), bc2 = (float)(1.0 - std::pow((double)b2, step));
-    for (int l = 0; l < layers(); l++) {
+    AdamLayers A;
+    A.n = layers();
+    int blocks = 0;
+    for (int l = 0; l < A.n; l++) {
         Layer& L = *L_[l];
-        const size_t nw = (size_t)L.out_p * L.in_p;
-        k_adam<<<grid_for(nw), 256, 0, s>>>(L.w, L.gw, L.mw, L.vw, L.live, nw, lr, b1, b2, eps, bc1, bc2, L.wb);
-        k_adam<<<grid_for(L.out), 256, 0, s>>>(L.b, L.gb, L.mb, L.vb, nullptr, (size_t)L.out, lr, b1, b2, eps, bc1,
-                                               bc2, nullptr);
-        k_transpose<<<dim3(L.in_p / 32, L.out_p / 32), dim3(32, 8), 0, s>>>(L.wb, L.out_p, L.in_p, L.wt);
-        launches_ += 3;
+        AdamLayer& a = A.l[l];
+        a = AdamLayer{L.w, L.gw, L.mw, L.vw, L.b, L.gb, L.mb, L.vb, L.live, L.wb, L.wt, L.in_p, L.out_p, L.out, blocks, 0};
+        blocks += (L.in_p / 32) * (L.out_p / 32);
+        a.bias0 = blocks;
+        blocks += (L.out + 255) / 256;
     }
+    k_adam<<<blocks, 256, 0, s>>>(A, lr, b1, b2, eps, bc1, bc2);
+    launches_++;
+    LCK(cudaGetLastError());
 }
 
 void LeafNet::get_params(int l, float* w, float* b) const {
@@ -717,7 +799,8 @@ void LeafNet::forward_host(const float* x, int rows, float* y) {
     DevBuf<int> idx_buf(rows);
     int* didx = idx_buf.p;
     LCK(cudaMemcpy(didx, idx.data(), rows * 4, cudaMemcpyHostToDevice));
-    k_gather_rows_bf16<<<rp, 256, 0, stream_>>>(X.p, didx, rows, d_.din, din_p_, x_);
+    k_gather_rows<<<dim3(rp, kGatherSplit), 256, 0, stream_>>>(X.p, nullptr, nullptr, didx, rows, d_.din, din_p_, d_.dout,
+                                                               dout_p_, x_, nullptr, nullptr);
     forward(x_, rp, y_, false, stream_);
     check(stream_);
     LCK(cudaMemcpy2D(y, d_.dout * 4, y_, dout_p_ * 4, d_.dout * 4, rows, cudaMemcpyDeviceToHost));
@@ -733,11 +816,14 @@ double LeafNet::gradients_host(const float* x, const float* t, const float* mask
     DevBuf<int> idx_buf(rows);
     int* didx = idx_buf.p;
     LCK(cudaMemcpy(didx, idx.data(), rows * 4, cudaMemcpyHostToDevice));
-    k_gather_rows_bf16<<<rp, 256, 0, stream_>>>(X.p, didx, rows, d_.din, din_p_, x_);
-    k_gather_rows_f32<<<rp, 256, 0, stream_>>>(T.p, didx, rows, d_.dout, dout_p_, t_);
-    k_gather_rows_f32<<<rp, 256, 0, stream_>>>(M.p, didx, rows, d_.dout, dout_p_, m_);
+    k_gather_rows<<<dim3(rp, kGatherSplit), 256, 0, stream_>>>(X.p, T.p, M.p, didx, rows, d_.din, din_p_, d_.dout, dout_p_,
+                                                               x_, t_, m_);
     forward(x_, rp, y_, true, stream_);
-    const double loss = backward(t_, m_, rp, rows, stream_);
+    LCK(cudaMemsetAsync(loss_, 0, sizeof(double), stream_));
+    backward(t_, m_, rp, rows, loss_, stream_);
+    double loss = 0.0;
+    LCK(cudaMemcpyAsync(&loss, loss_, sizeof(double), cudaMemcpyDeviceToHost, stream_));
+    check(stream_);
     return loss;
 }
 
@@ -746,27 +832,30 @@ void LeafNet::train_host(const float* x, const float* t, const float* mask, int 
     if (n <= 0 || epochs <= 0 || batch <= 0 || batch % 128) throw Error("invalid argument: training sizes");
     ensure_rows(batch);
     DevTable X(x, (size_t)n * d_.din), T(t, (size_t)n * d_.dout), M(mask, (size_t)n * d_.dout);
-    DevBuf<int> idx_buf(batch);
-    int* didx = idx_buf.p;
+    const int nb = std::max(1, n / batch);  // whole batches (one short batch when n < batch)
+    DevBuf<int> idx_buf(n);
+    DevBuf<double> loss_buf(nb);  // a step's loss each, read at the epoch's end: the steps need no host in between
+    std::vector<double> loss(nb);
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     uint64_t s = seed * 0x9E3779B97F4A7C15ull + 1;
     if (!s) s = 1;
     for (int ep = 0; ep < epochs; ep++) {
         for (int i = n - 1; i > 0; i--) std::swap(order[i], order[(size_t)(xs_next(s) % (uint64_t)(i + 1))]);
-        double sum = 0.0;
-        const int nb = std::max(1, n / batch);  // whole batches (one short batch when n < batch)
+        LCK(cudaMemcpyAsync(idx_buf.p, order.data(), (size_t)n * 4, cudaMemcpyHostToDevice, stream_));
+        LCK(cudaMemsetAsync(loss_buf.p, 0, (size_t)nb * sizeof(double), stream_));
         for (int bi = 0; bi < nb; bi++) {
             const int b0 = bi * batch, rows = std::min(batch, n - b0);
-            LCK(cudaMemcpyAsync(didx, order.data() + b0, rows * 4, cudaMemcpyHostToDevice, stream_));
-            k_gather_rows_bf16<<<batch, 256, 0, stream_>>>(X.p, didx, rows, d_.din, din_p_, x_);
-            k_gather_rows_f32<<<batch, 256, 0, stream_>>>(T.p, didx, rows, d_.dout, dout_p_, t_);
-            k_gather_rows_f32<<<batch, 256, 0, stream_>>>(M.p, didx, rows, d_.dout, dout_p_, m_);
+            k_gather_rows<<<dim3(batch, kGatherSplit), 256, 0, stream_>>>(X.p, T.p, M.p, idx_buf.p + b0, rows, d_.din, din_p_,
+                                                                          d_.dout, dout_p_, x_, t_, m_);
             forward(x_, batch, y_, true, stream_);
-            sum += backward(t_, m_, batch, rows, stream_);
+            backward(t_, m_, batch, rows, loss_buf.p + bi, stream_);
             adam(lr, ++adam_t_, stream_);
         }
+        LCK(cudaMemcpyAsync(loss.data(), loss_buf.p, (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, stream_));
         check(stream_);
+        double sum = 0.0;
+        for (double x : loss) sum += x;
         if (losses) losses[ep] = (float)(sum / std::max(nb, 1));
     }
 }
@@ -846,24 +935,38 @@ __global__ void k_leaf_err(LeafDev L) {
     const float e = block_sum(acc, red);
     if (threadIdx.x == 0) L.err[row] = e;
 }
-// one block per leaf: player p's values, summed over the turn cards
-__global__ void k_leaf_scatter(LeafDev L, int p, float* cfv, size_t stride) {
-    const int li = blockIdx.x;
+// player p's values of a leaf, summed over the turn cards in order; 64 hands
+// of one leaf per block, four threads a hand load its cards' rows (one block
+// per leaf walking the cards took 43 us)
+constexpr int kScatterHands = 64, kScatterParts = 4;
+__global__ void __launch_bounds__(kScatterHands* kScatterParts) k_leaf_scatter(LeafDev L, int p, float* cfv,
+                                                                               size_t stride, int chunks) {
+    constexpr int N = 13;  // 4 x 13 = 52 cards
+    __shared__ float s_v[52][kScatterHands];
+    const int li = (int)blockIdx.x / chunks, hl = threadIdx.x % kScatterHands, part = threadIdx.x / kScatterHands;
+    const int h = ((int)blockIdx.x % chunks) * kScatterHands + hl;
     const LeafItem lf = L.leaves[li];
     const float inv = 1.0f / 45.0f;
-    for (int h = threadIdx.x; h < L.nh[p]; h += blockDim.x) {
-        const uint64_t hm = L.hmask[p][h];
-        const int cb = L.combo[p][h];
-        float acc = 0.0f;
-        for (int j = 0; j < L.ncards; j++) {
-            const int c = L.cards[j];
-            if ((hm >> c) & 1ull) continue;
+    const bool on = h < L.nh[p];
+    const uint64_t hm = on ? L.hmask[p][h] : 0ull;
+    const int cb = on ? L.combo[p][h] : 0;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const int j = part * N + k;
+        float v = 0.0f;  // a card the hand holds adds nothing
+        if (on && j < L.ncards && !((hm >> L.cards[j]) & 1ull)) {
             const int row = li * L.ncards + j;
             const float yv = L.y[(size_t)row * L.dout_p + p * 1326 + cb] - 0.5f * L.err[row];
-            acc += yv * lf.pot * L.mass[row * 2 + (1 - p)];
+            v = yv * lf.pot * L.mass[row * 2 + (1 - p)];
         }
-        cfv[(size_t)lf.cslot * stride + h] = acc * inv;
+        s_v[j][hl] = v;
     }
+    __syncthreads();
+    if (part != 0 || !on) return;
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 52; j++) acc += s_v[j][hl];
+    cfv[(size_t)lf.cslot * stride + h] = acc * inv;
 }
 template <class T>
 T* dcopy(const T* h, size_t n) {
@@ -945,7 +1048,8 @@ void LeafEvaluator::run(int p, const float* reach0, size_t rstr0, const float* r
     k_leaf_gather<<<rows_, 256, 0, s>>>(L);
     net_->forward_device(x_, rows_p_, y_, s);
     k_leaf_err<<<rows_, 256, 0, s>>>(L);
-    k_leaf_scatter<<<nleaves_, 256, 0, s>>>(L, p, cfv, cfv_stride);
+    const int chunks = (nh_[p] + kScatterHands - 1) / kScatterHands;
+    k_leaf_scatter<<<nleaves_ * chunks, kScatterHands * kScatterParts, 0, s>>>(L, p, cfv, cfv_stride, chunks);
     LCK(cudaGetLastError());
 }
 

@@ -76,7 +76,8 @@ class LeafNet {
     struct Layer;
     void ensure_rows(int rows_pad);
     void forward(const __nv_bfloat16* x, int rows_pad, float* y, bool keep, cudaStream_t s);
-    double backward(const float* t, const float* mask, int rows_pad, int rows, cudaStream_t s);
+    // adds the masked mean squared error to *loss (device), leaves the gradients on the device
+    void backward(const float* t, const float* mask, int rows_pad, int rows, double* loss, cudaStream_t s);
     void adam(float lr, int step, cudaStream_t s);
     void check(cudaStream_t s);
     LeafNetDims d_;
@@ -89,7 +90,8 @@ class LeafNet {
     unsigned* err_ = nullptr;
     int adam_t_ = 0;
     uint32_t launches_ = 0;
-    cudaStream_t stream_ = nullptr;
+    cudaStream_t stream_ = nullptr, side_ = nullptr;  // side_: weight gradients of a backward pass
+    cudaEvent_t ev_ = nullptr;
 };
 
 // The turn-leaf inputs and outputs of a depth-limited flop plan.  Inputs per
