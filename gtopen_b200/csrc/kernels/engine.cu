@@ -126,6 +126,7 @@ struct EngineImpl {
     uint32_t* fold_slots[2] = {nullptr, nullptr};  // per traverser the opponent's reach slot of each
     ChanceItem* chance = nullptr;
     XNode* xnodes[2] = {nullptr, nullptr};
+    XNode* xpacked[2] = {nullptr, nullptr};  // the same blocks packed in order (export of an engine that holds few)
     std::vector<XNode> hx[2];
     void* lock_buf = nullptr;
     float* staging = nullptr;  // device f32 image of one arena in the reference layout
@@ -810,6 +811,26 @@ static void setup_shows(EngineImpl& E) {
         set_smem(show_group_kernel(sg.shape[q]), show_group_smem(sg.shape[q], sg.max_sorted[q], P.nh[q]));
 }
 
+// Zeros, by several threads; pages that hold zeros already are only read, so
+// a fresh buffer's pages are not materialised.
+static void zero_fill(void* dst, size_t bytes) {
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int nt = (int)std::max(1u, std::min(8u, hw ? hw : 1u));
+    const size_t pages = (bytes + 4095) / 4096, per = (pages + nt - 1) / nt;
+    auto run = [=](int w) {
+        unsigned char* base = (unsigned char*)dst;
+        for (size_t k = std::min(pages, w * per); k < std::min(pages, (w + 1) * per); k++) {
+            unsigned char* q = base + k * 4096;
+            const size_t n = std::min<size_t>(4096, bytes - k * 4096);
+            if (q[0] != 0 || std::memcmp(q, q + 1, n - 1) != 0) std::memset(q, 0, n);
+        }
+    };
+    std::vector<std::thread> ts;
+    for (int w = 1; w < nt; w++) ts.emplace_back(run, w);
+    run(0);
+    for (auto& t : ts) t.join();
+}
+
 // --------------------------------------------------------------- GpuEngine
 GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine) : GpuEngine(host, fmt, engine, 0, 1, nullptr) {}
 
@@ -1188,6 +1209,31 @@ void GpuEngine::root_cfv(int p, int mode, float* out) {
 
 void GpuEngine::export_arena(int which, int p, float* out) {
     EngineImpl& E = *d_;
+    const size_t len = E.spot->tree.data_size[p], held = E.plan.visited_action_elems[p];
+    if (held * 8 <= len && len * 4 >= 2 * kPinChunk && (which != kPreds || E.pcfr)) {
+        // a depth-limited solve or a shard holds a fraction of the arena: only
+        // its blocks cross the bus, packed; the rest of the output is zeroed
+        const int nh = E.plan.nh[p];
+        if (!E.xpacked[p]) {
+            std::vector<XNode> xs(E.hx[p]);
+            uint64_t at = 0;
+            for (XNode& x : xs) {
+                x.host_off = at;
+                at += (uint64_t)x.na * nh;
+            }
+            E.xpacked[p] = dupload(xs, E.owned, &E.bytes);
+        }
+        decode_blocks(which, p, E.xpacked[p]);
+        std::vector<float> tmp(held);
+        E.d2h_large(tmp.data(), E.staging, held * 4);
+        zero_fill(out, len * 4);
+        size_t at = 0;
+        for (const XNode& x : E.hx[p]) {
+            std::memcpy(out + x.host_off, tmp.data() + at, (size_t)x.na * nh * 4);
+            at += (size_t)x.na * nh;
+        }
+        return;
+    }
     fill_staging(which, p);
     E.d2h_large(out, E.staging, E.spot->tree.data_size[p] * 4);
 }
@@ -1196,21 +1242,26 @@ void GpuEngine::export_arena(int which, int p, float* out) {
 void GpuEngine::fill_staging(int which, int p) {
     EngineImpl& E = *d_;
     CK(cudaMemsetAsync(E.staging, 0, E.staging_len * 4, E.stream));
+    decode_blocks(which, p, E.xnodes[p]);
+}
+// The device's blocks decoded into `staging` at the offsets of xs.
+void GpuEngine::decode_blocks(int which, int p, const XNode* xs) {
+    EngineImpl& E = *d_;
     const unsigned nb = (unsigned)E.plan.n_anodes[p];
     void* src = which == kRegrets ? E.ar.reg[p] : which == kStrategy ? E.ar.str[p] : E.ar.pred[p];
     if (nb && src) {
         if (E.fmt == kFmtF32) {
-            k_to_host<float><<<nb, kThreads, 0, E.stream>>>((const float*)src, E.staging, E.xnodes[p], E.plan.nh[p]);
+            k_to_host<float><<<nb, kThreads, 0, E.stream>>>((const float*)src, E.staging, xs, E.plan.nh[p]);
         } else if (E.fmt == kFmtFP8) {
             const float* sc = which == kRegrets ? E.ar.rscale[p] : which == kStrategy ? E.ar.sscale[p] : E.ar.pscale[p];
-            k_decode_fp8_to_host<<<nb, kThreads, 0, E.stream>>>((const uint8_t*)src, sc, E.staging, E.xnodes[p],
+            k_decode_fp8_to_host<<<nb, kThreads, 0, E.stream>>>((const uint8_t*)src, sc, E.staging, xs,
                                                                  E.plan.nh[p]);
         } else if (which == kStrategy) {
             k_decode_to_host<uint16_t><<<nb, kThreads, 0, E.stream>>>((const uint16_t*)src, E.ar.sscale[p], E.staging,
-                                                                       E.xnodes[p], E.plan.nh[p], 65535.0f);
+                                                                       xs, E.plan.nh[p], 65535.0f);
         } else {
             const float* sc = which == kRegrets ? E.ar.rscale[p] : E.ar.pscale[p];
-            k_decode_to_host<int16_t><<<nb, kThreads, 0, E.stream>>>((const int16_t*)src, sc, E.staging, E.xnodes[p],
+            k_decode_to_host<int16_t><<<nb, kThreads, 0, E.stream>>>((const int16_t*)src, sc, E.staging, xs,
                                                                       E.plan.nh[p], 32767.0f);
         }
         CK(cudaGetLastError());

@@ -100,6 +100,7 @@ class GpuEngine {
     // success.  Returns the element count written to out.
     size_t read_node_static(int which, uint32_t node, float* out, size_t out_len);
     void fill_staging(int which, int p);
+    void decode_blocks(int which, int p, const struct XNode* xs);
     // Average strategy of one action node the device holds (reference layout
     // [action * nh + hand]), by the rule the evaluation sweeps use.
     void node_average_strategy(uint32_t node, float* out);
