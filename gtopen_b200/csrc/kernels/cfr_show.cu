@@ -20,7 +20,7 @@
 //   * The fewest threads whose lanes hold the scan, then the largest G: the
 //     per-warp work (shuffles, carries, address set-up) is paid by fewer
 //     warps.  Measured, ms per iteration for both sweeps (threads x G):
-//     28 v 23 hands 64x8 0.077, 128x8 0.111, 64x2 0.199; 64 v 39 hands 64x8
+//     28 v 23 hands 32x8 0.070, 64x8 0.080, 128x8 0.111, 64x2 0.199; 64 v 39 hands 64x8
 //     0.246, 128x8 0.288, 64x2 0.443; 243 v 321 64x2 2.35, 128x4 2.43, 256x8
 //     2.70; 470 v 647 128x2 1.45, 256x4 1.65, 512x8 2.12.
 // Showdowns of one iteration before (two at a time, one launch per level,
@@ -504,6 +504,9 @@ bool with_show(const ShowShape& sh, F f) {
     using C8 = std::integral_constant<int, 8>;
     using C4 = std::integral_constant<int, 4>;
     using C2 = std::integral_constant<int, 2>;
+    if (sh.threads == 32 && sh.group == 8) return by_k(C8{}, std::integral_constant<int, 32>{});
+    if (sh.threads == 32 && sh.group == 4) return by_k(C4{}, std::integral_constant<int, 32>{});
+    if (sh.threads == 32 && sh.group == 2) return by_k(C2{}, std::integral_constant<int, 32>{});
     if (sh.threads == 64 && sh.group == 8) return by_k(C8{}, std::integral_constant<int, 64>{});
     if (sh.threads == 64 && sh.group == 4) return by_k(C4{}, std::integral_constant<int, 64>{});
     if (sh.threads == 64 && sh.group == 2) return by_k(C2{}, std::integral_constant<int, 64>{});
@@ -514,7 +517,7 @@ bool with_show(const ShowShape& sh, F f) {
 }  // namespace
 
 bool show_shape(int group, int max_sorted, ShowShape& sh) {
-    for (int threads = 64; threads <= (group == 2 ? 256 : 64); threads *= 2) {
+    for (int threads = 32; threads <= (group == 2 ? 256 : 64); threads *= 2) {
         const int rows = threads / (group / 2), k = (3 * max_sorted + rows - 1) / rows;
         sh = {group, threads, k <= 4 ? 4 : (k + 3) / 4 * 4};
         if (sh.chunk <= 16) return true;

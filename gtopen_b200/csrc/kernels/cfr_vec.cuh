@@ -42,6 +42,15 @@
 namespace gtob {
 namespace {
 
+// CTAs of 128 threads an SM must hold, for the forms that carry the large
+// launches (V = 4, nodes of at most 4 actions): they wait for HBM, and more
+// warps in flight are worth the spills of the rare 4-action body.  Down 16
+// (32 registers), opponent 14, f32 update 8 (64); the quantised update's CTAs
+// 56 registers a thread.  Registers as the compiler takes them -> capped, ms
+// per iteration: 243 v 321 hands f32 down 0.96 -> 0.81, up 3.63 -> 3.03 (f32
+// update 10 CTAs: 3.32); 470 v 647 16-bit down 0.50 -> 0.42, up 1.89 -> 1.59
+// (64 registers: 1.67, 48: 1.64).
+constexpr int kVDownCtas = 16, kVOppCtas = 14, kVMineCtas = 8, kVQuantRegs = 56;
 constexpr int kVMaxWarps = 32;
 constexpr uint64_t kVFillWarps = 148 * 16;  // warps that fill the device
 
@@ -261,7 +270,7 @@ __device__ __forceinline__ void v_down_node(const Dev& d, const Arenas& ar, cons
         if (it.rs[k] != kNoSlot) out[k].store(pick(d.reach, a) + (size_t)it.rs[k] * pick(d.rstr, a) + i0);
 }
 template <int FMT, int SRC, int V, int KA>
-__global__ void __launch_bounds__(128) kv_down(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn) {
+__global__ void __launch_bounds__(128, V == 4 && KA == 4 && SRC == kVRegret ? kVDownCtas : 1) kv_down(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn) {
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
     if (n >= count) return;
     const SNodeT<KA>& it = nodes[n];
@@ -515,7 +524,7 @@ __device__ __forceinline__ void v_mine_node(const Dev& d, const Arenas& ar, cons
 // Nodes whose hands do not depend on one another (the opponent's nodes,
 // evaluation sweeps, f32 arenas): one warp per 32 V hands, wn warps per node.
 template <int V, int KA>
-__global__ void __launch_bounds__(128) kv_up_opp(Dev d, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn, int p) {
+__global__ void __launch_bounds__(128, V == 4 && KA == 4 ? kVOppCtas : 1) kv_up_opp(Dev d, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn, int p) {
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
     if (n >= count) return;
     const SNodeT<KA>& it = nodes[n];
@@ -532,7 +541,7 @@ __global__ void __launch_bounds__(128) kv_up_opp(Dev d, const SNodeT<KA>* nodes,
     }
 }
 template <int FMT, int EVAL, bool PRED, int V, int KA>
-__global__ void __launch_bounds__(128) kv_up_mine(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn,
+__global__ void __launch_bounds__(128, V == 4 && KA == 4 && !EVAL && !PRED ? kVMineCtas : 1) kv_up_mine(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn,
                                                   int p, int mode) {
     static_assert(EVAL || FMT == kDevF32, "a quantised update needs the node's maxima");
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
@@ -550,9 +559,10 @@ __global__ void __launch_bounds__(128) kv_up_mine(Dev d, Arenas ar, const SNodeT
         V_CASE(1) V_CASE(2) V_CASE(3) V_CASE(4) V_CASE(5) V_CASE(6) V_CASE(7) V_CASE(8)
     }
 }
-// Updates of quantised arenas: one warp per node (WARP), or one CTA.
+// Updates of quantised arenas: one warp per node (WARP), or one CTA of at most
+// 11 warps (V = 4) or 21 (V = 2: 96 registers a thread still fit an SM).
 template <int FMT, bool PRED, bool WARP, int V, int KA>
-__global__ void __launch_bounds__(WARP ? 128 : (1326 + 32 * V - 1) / (32 * V) * 32)
+__global__ void __maxnreg__(WARP ? 168 : V == 2 ? 96 : KA == 4 ? kVQuantRegs : 160)
     kv_up_quant(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, int p) {
     __shared__ uint32_t red[WARP ? 1 : 3 * kVMaxWarps];
     const uint32_t n = WARP ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
