@@ -270,7 +270,7 @@ __device__ __forceinline__ void v_down_node(const Dev& d, const Arenas& ar, cons
         if (it.rs[k] != kNoSlot) out[k].store(pick(d.reach, a) + (size_t)it.rs[k] * pick(d.rstr, a) + i0);
 }
 template <int FMT, int SRC, int V, int KA>
-__global__ void __launch_bounds__(128, V == 4 && KA == 4 && SRC == kVRegret ? kVDownCtas : 1) kv_down(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn) {
+__global__ void __launch_bounds__(128, V != 4 || KA != 4 || SRC == kVPredicted ? 1 : SRC == kVRegret ? kVDownCtas : 10) kv_down(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn) {
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
     if (n >= count) return;
     const SNodeT<KA>& it = nodes[n];
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(128, V == 4 && KA == 4 ? kVOppCtas : 1) kv_up_
     }
 }
 template <int FMT, int EVAL, bool PRED, int V, int KA>
-__global__ void __launch_bounds__(128, V == 4 && KA == 4 && !EVAL && !PRED ? kVMineCtas : 1) kv_up_mine(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn,
+__global__ void __launch_bounds__(128, V == 4 && KA == 4 && !PRED ? kVMineCtas : 1) kv_up_mine(Dev d, Arenas ar, const SNodeT<KA>* nodes, uint32_t count, uint32_t wn,
                                                   int p, int mode) {
     static_assert(EVAL || FMT == kDevF32, "a quantised update needs the node's maxima");
     const uint32_t w = blockIdx.x * 4 + (threadIdx.x >> 5), n = w / wn;
