@@ -442,8 +442,8 @@ class GpuSolver:
     """gpu/mod.rs GpuSolver: device buffers, CUDA-graph iterations, BR checks, syncs."""
 
     def __init__(self, solver, device_format=None, engine="staged"):
-        """engine: "staged" (default: one CTA per node, its data staged in
-        shared memory by bulk copies; showdowns batched by river board),
+        """engine: "staged" (default: a node's hands in registers, warps or
+        CTAs per node; a sweep's showdowns and folds one launch each),
         "fused" (terminals evaluated inside their parents' kernels, f64
         terminal sums), "plain" (one launch per node kind and level, f64
         terminal sums), "fused32" (fused, f32 terminal sums) or "warp" (one

@@ -1,6 +1,6 @@
-// Staged node kernels (the STAGED engine): one CTA per node stages every
-// vector and arena block the node needs in shared memory with bulk
-// asynchronous copies -- the TMA unit's non-tensor mode, cp.async.bulk --
+// Staged node functions (the batched kernel's and, in part, the river
+// programs'): one CTA per node stages every vector and arena block the node
+// needs in shared memory with bulk asynchronous copies -- the TMA unit's non-tensor mode, cp.async.bulk --
 // that complete on one mbarrier, then computes from shared memory and writes
 // its results with 16-byte stores.  All of a node's HBM reads are in flight
 // at once (one round trip instead of one per hand chunk and arena field), and

@@ -4,10 +4,15 @@
 // vectors level by level, then an up sweep folding counterfactual values back
 // to the root with the DCFR / CFR+ / PCFR+ regret and strategy-sum update --
 // the work split of the reference's gpu/kernels.cu and gpu/mod.rs:622-841,
-// re-designed for B200 (device code in cfr_kernels.cuh):
+// re-designed for B200:
 //   * work items carry precomputed slots (plan.hpp); reach and cfv vectors
 //     live in compact slots;
-//   * FUSED engine (default): fold and showdown children are evaluated in
+//   * STAGED engine (default): the vector kernels (cfr_vec.cuh) for action
+//     nodes, one launch per sweep for all showdowns and one for all folds
+//     (cfr_show.cu), a level's launches side by side; its records also feed
+//     the batched kernel and the river programs, which stage nodes in shared
+//     memory (cfr_staged.cuh, cfr_batch.cuh, cfr_river.cuh);
+//   * FUSED engine: fold and showdown children are evaluated in
 //     shared memory by their parent's up-sweep kernel (all-in runouts by the
 //     river chance node's kernel), so terminals -- two thirds of all nodes --
 //     never write or read a vector in HBM and need no launches of their own;
@@ -1813,6 +1818,7 @@ uint64_t estimate_vram(const Spot& spot) {  // same role as game.rs:365-373, for
     uint64_t b = P.n_cslots * (uint64_t)P.nh_max * 4 + P.n_rslots[0] * (uint64_t)P.nh[0] * 4 +
                  P.n_rslots[1] * (uint64_t)P.nh[1] * 4;
     b += (P.arena_len[0] + P.arena_len[1]) * 2 * 4;
+    for (const ActItem& a : P.act) b += a.nterm * sizeof(FoldSum);
     return b + 512ull * 1024 * 1024;
 }
 bool vram_info_mb(uint64_t* free_mb, uint64_t* total_mb) {

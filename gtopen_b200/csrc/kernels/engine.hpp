@@ -56,8 +56,8 @@ class GpuEngine {
     // per terminal level, f64 sums), kEngineFused32 (fused, f32 sums as the
     // reference GPU kernels), kEngineWarp (one warp per action node, fold
     // children evaluated in place by the warp, showdowns one CTA each; f64),
-    // kEngineStaged (one CTA per node staging its blocks and vectors in shared
-    // memory with bulk copies; fold children in place; exact sums),
+    // kEngineStaged (a node's hands in registers, a warp or a CTA per node; a
+    // sweep's showdowns and folds one launch each; exact sums),
     // kEngineStagedRiver (the staged engine with river betting rounds solved
     // by river programs, cfr_river.cuh).
     GpuEngine(const HostSolver& host, int fmt, int engine = 0);

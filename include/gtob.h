@@ -44,13 +44,13 @@ extern "C" {
                                    regrets may round differently than the CPU engine) */
 #define GTOB_ENGINE_WARP 3      /* one warp per action node with its fold child evaluated
                                    in the warp; showdowns one CTA each; f64 terminal sums */
-#define GTOB_ENGINE_STAGED 4    /* one CTA per node staging its arena blocks and vectors in
-                                   shared memory with bulk copies; fold children in place;
-                                   exact terminal sums (nodes with more than 4 actions: the
-                                   warp engine's kernels) */
+#define GTOB_ENGINE_STAGED 4    /* the default: a node's hands in registers, a warp or a CTA per
+                                   node; a sweep's showdowns and its folds' card sums one
+                                   launch each; exact terminal sums (nodes with more than 8
+                                   actions: the warp engine's kernels) */
 #define GTOB_ENGINE_STAGED_RIVER 5 /* the staged engine with every river betting round solved by
                                    one CTA walking it depth first (river programs); the same
-                                   results bit for bit, slower on this device (see DESIGN) */
+                                   results bit for bit, slower on this device */
 #define GTOB_ARENA_REGRETS 0
 #define GTOB_ARENA_STRATEGY 1
 #define GTOB_ARENA_PREDICTIONS 2

@@ -94,3 +94,64 @@ def test_suit_symmetric_flop():
     cfg = W.iso_spot()
     _equal(cfg)
     _equal(cfg, "compressed", "i16sr")
+
+
+def test_export_of_an_engine_that_holds_few_nodes():
+    """A depth-limited solve's export: its nodes' average strategies, zeros
+    elsewhere (only the held blocks are read back)."""
+    cfg = W.flop_spot(g.evaluate7, seed=6, bet=("50",), raise_=("2.5x",), max_raises=1, pot=100, stack=330,
+                      frac=(0.15, 0.2))
+    spot = g.Spot(cfg)
+    host = g.Solver(spot)
+    gpu = g.dl_gpu_solver(host, g.LeafNet(2705, 128, 1, 2652, seed=2))
+    gpu.iterate(3)
+    t = spot.tree()
+    _, _, _, visited = g.dl_plan(spot)
+    for p in (0, 1):
+        assert spot.data_size[p] * 4 >= 8 << 20
+        sums = gpu.export_arena(1, p)
+        held = np.zeros(spot.data_size[p], bool)
+        for n in np.nonzero(visited.astype(bool) & (t["kind"] == 0) & (t["player"] == p))[0]:
+            na, off = int(t["nchild"][n]), int(t["data_off"][n])
+            held[off:off + na * spot.nh[p]] = True
+            s = np.maximum(sums[off:off + na * spot.nh[p]].reshape(na, -1), 0).astype(np.float64)
+            total = s.sum(0)
+            want = np.where(total > 1e-12, s / np.where(total > 0, total, 1), 1.0 / na)
+            got = g.node_strategy(gpu, int(n), na, p)
+            assert np.abs(got - want).max() <= 2e-7  # one f32 rounding of the same quotient
+        assert held.any() and not sums[~held].any()
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 128, 64), (128, 256, 192), (256, 2688, 128), (1024, 1024, 64), (1024, 2048, 64),
+                                   (2048, 2048, 64)])
+def test_product_tile_widths(m, n, k):
+    """The tcgen05 product at shapes that take each tile width (32 to 256
+    columns): f32 accumulation against f64, 1e-5 of sum |a||b|."""
+    rng = np.random.default_rng(m + n)
+    a, b = (rng.normal(0, 1, (r, k)).astype(np.float32) for r in (m, n))
+    bits = [(x.view(np.uint32) >> 16).astype(np.uint16) for x in (a, b)]
+    a, b = (((x.astype(np.uint32)) << 16).view(np.float32).astype(np.float64) for x in bits)
+    c = g.gemm_bf16(*bits)
+    assert np.all(np.abs(c - a @ b.T) <= 1e-5 * (np.abs(a) @ np.abs(b).T) + 1e-6)
+
+
+def test_one_adam_step():
+    """One training step on one batch against Adam's formula on the gradients
+    the network reports (padded, odd dimensions; every layer, weights and
+    biases).  The first step moves an entry by lr g / (|g| + eps'): insensitive
+    to the batch order's rounding where |g| is well above eps."""
+    dims, n, lr = (70, 130, 2, 40), 128, 1e-2
+    rng = np.random.default_rng(5)
+    x, t = rng.normal(0, 1, (n, 70)).astype(np.float32), rng.normal(0, 1, (n, 40)).astype(np.float32)
+    m = (rng.random((n, 40)) < 0.8).astype(np.float32)
+    a, b = g.LeafNet(*dims, seed=3), g.LeafNet(*dims, seed=3)
+    loss = a.gradients(x, t, m)
+    losses = b.train(x, t, m, epochs=1, batch=n, lr=lr, seed=1)
+    assert abs(losses[0] - loss) <= 1e-5 * loss
+    for layer in range(dims[2] + 1):
+        for w, gr, got in zip(a.params(layer), a.grads(layer), b.params(layer)):
+            gr = gr.astype(np.float64)
+            want = w - lr * gr / (np.abs(gr) + 1e-8)
+            big = np.abs(gr) > 1e-5
+            assert big.any() and np.abs(got - want)[big].max() <= 1e-2 * lr
+            assert np.abs(got - w).max() <= lr * 1.001
