@@ -760,7 +760,7 @@ static void setup_shows(EngineImpl& E) {
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     std::vector<uint32_t> per(P.num_slots, 0);
-    for (const ShowItem& x : P.show) per[x.slot]++;
+    for (const ShowBatch& b : P.show_batch) per[b.slot] += b.count;
     ShowGroups sg;
     for (int q = 0; q < 2; q++)
         for (uint32_t c : P.sorted_cnt[q]) sg.max_sorted[q] = std::max(sg.max_sorted[q], (int)c);
@@ -786,28 +786,30 @@ static void setup_shows(EngineImpl& E) {
     CK(cudaGetLastError());
     auto group = [&](bool upper_only) {
         ShowGroups g = sg;
+        // the level-ordered batches hold one slot each: whole runs move
         std::vector<uint32_t> at(P.num_slots + 1, 0);
         auto each = [&](auto f) {
             for (size_t l = 0; l < P.show_batch_span.size(); l++) {
                 const Span s = upper_only ? P.show_batch_span_upper[l] : P.show_batch_span[l];
-                for (uint32_t b = s.start; b < s.start + s.count; b++)
-                    for (uint32_t k = 0; k < P.show_batch[b].count; k++) f(P.show[P.show_batch[b].start + k]);
+                for (uint32_t b = s.start; b < s.start + s.count; b++) f(P.show_batch[b]);
             }
         };
-        each([&](const ShowItem& x) { at[x.slot + 1]++; });
+        each([&](const ShowBatch& b) { at[b.slot + 1] += b.count; });
         const uint32_t G = (uint32_t)g.shape[0].group;
-        std::vector<uint32_t> slot_of;  // per batch
+        uint64_t items = 0;
+        for (uint32_t s = 0; s < P.num_slots; s++) items += (at[s + 1] + G - 1) / G * G;
+        PodVec<ShowItem> it(items);
         for (uint32_t s = 0; s < P.num_slots; s++) {
-            const uint32_t nb = (at[s + 1] + G - 1) / G;
-            slot_of.insert(slot_of.end(), nb, s);
-            at[s + 1] = at[s] + nb * G;
+            const uint32_t n = at[s + 1], e = (n + G - 1) / G * G;
+            for (uint32_t k = n; k < e; k++) it[at[s] + k] = ShowItem{kNoSlot, {0, 0}, s, 0.0f, 0.0f, 0.0f, 0};
+            at[s + 1] = at[s] + e;
         }
-        PodVec<ShowItem> it(slot_of.size() * G);
-        for (size_t b = 0; b < slot_of.size(); b++)
-            for (uint32_t k = 0; k < G; k++) it[b * G + k] = ShowItem{kNoSlot, {0, 0}, slot_of[b], 0.0f, 0.0f, 0.0f, 0};
-        each([&](const ShowItem& x) { it[at[x.slot]++] = x; });
+        each([&](const ShowBatch& b) {
+            std::copy(P.show.begin() + b.start, P.show.begin() + b.start + b.count, it.begin() + at[b.slot]);
+            at[b.slot] += b.count;
+        });
         g.items = dupload(it, O, &B);
-        g.count = (uint32_t)slot_of.size();
+        g.count = (uint32_t)(items / G);
         return g;
     };
     E.shows = group(false);
@@ -948,17 +950,29 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     if (E.warp) E.warp_smem = (size_t)kWarps * d.nh_pad * sizeof(float);
     if (E.vec) {
         // node records, packed hand words; folds numbered in record order
-        std::vector<uint32_t> fold_no(P.act.size(), 0), fs[2];
-        for (size_t k = 0; k < P.act.size(); k++) {
-            const ActItem& a = P.act[k];
-            if (!a.nterm) continue;  // in-place terminals: folds only
-            fold_no[k] = (uint32_t)fs[0].size();
-            for (uint32_t c = 0; c < a.na; c++)
-                if (P.crefs[a.cref + c].kind == kChildFold) {
-                    fs[a.actor].push_back(a.oslot);                        // the traverser folds: the opponent's reach here
-                    fs[1 - a.actor].push_back(P.crefs[a.cref + c].rslot);  // the opponent does: its reach at the fold
-                }
-        }
+        const size_t na = P.act.size(), step = 65536, chunks = (na + step - 1) / step;
+        std::vector<uint32_t> fold_no(na, 0), base(chunks + 1, 0);
+        PodVec<uint32_t> fs[2];
+        parallel_for(chunks, [&](size_t c) {  // an action node's in-place terminals: its fold child
+            for (size_t k = c * step; k < std::min(na, (c + 1) * step); k++) base[c + 1] += P.act[k].nterm;
+        });
+        for (size_t c = 0; c < chunks; c++) base[c + 1] += base[c];
+        fs[0].resize(base[chunks]);
+        fs[1].resize(base[chunks]);
+        parallel_for(chunks, [&](size_t c) {
+            uint32_t at = base[c];
+            for (size_t k = c * step; k < std::min(na, (c + 1) * step); k++) {
+                const ActItem& a = P.act[k];
+                if (!a.nterm) continue;
+                for (uint32_t j = 0; j < a.na; j++)
+                    if (P.crefs[a.cref + j].kind == kChildFold) {
+                        fold_no[k] = at;
+                        fs[a.actor][at] = a.oslot;                        // the traverser folds: the opponent's reach here
+                        fs[1 - a.actor][at] = P.crefs[a.cref + j].rslot;  // the opponent does: its reach at the fold
+                        at++;
+                    }
+            }
+        });
         E.nfolds = (uint32_t)fs[0].size();
         for (int q = 0; q < 2; q++) {
             E.fold_slots[q] = dupload(fs[q], O, &B);
