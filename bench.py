@@ -160,11 +160,11 @@ def barrier(world):
 # default); f32; fp8 = f32 host arenas, FP8 E4M3 device arenas (precision study)
 # DRAM bytes (read + write) of one CFR iteration, summed over every launch of
 # an iteration in a one-pass ncu capture (dram__bytes_read.sum +
-# dram__bytes_write.sum).  flop_narrow is captured directly (6.690 GB per
-# iteration, profiles/staged_engine_flop_narrow_launches.md); the flop's figure
-# is that capture scaled by the ratio of algorithmic bytes (127.48 / 3.946 GB).
-# Only for the configurations captured.
-MEASURED_TRAFFIC = {("flop_narrow", "i16sr", "staged"): 6.690e9, ("flop", "i16sr", "staged"): 216.1e9}
+# dram__bytes_write.sum).  flop_narrow is captured directly (5.746 GB per
+# iteration, profiles/vector_kernels_ncu.md); the flop's figure is that capture
+# scaled by the ratio of algorithmic bytes (127.48 / 3.946 GB).  Only for the
+# configurations captured.
+MEASURED_TRAFFIC = {("flop_narrow", "i16sr", "staged"): 5.746e9, ("flop", "i16sr", "staged"): 185.6e9}
 
 # i16sr = i16/u16 arenas whose update requantises with stochastic rounding
 # (the default: store.rs's round-to-nearest stalls on the flop workload)
