@@ -268,6 +268,7 @@ struct EngineImpl {
         CK(cudaMemcpy(base, off[0].data(), b0, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(base + b0, off[1].data(), b1, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(base + b0 + b1, sig.data(), bs, cudaMemcpyHostToDevice));
+        CK(cudaStreamSynchronize(0));  // before the engine's own (non-blocking) stream reads them
         d.lock_off[0] = (const long long*)base;
         d.lock_off[1] = (const long long*)(base + b0);
         d.lock_sig = (const float*)(base + b0 + b1);
@@ -1099,6 +1100,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
                 const size_t len = sp.tree.data_size[q];
                 if (ha->kind == 1) CK(cudaMemcpy(E.staging, ha->qi.data(), len * 2, cudaMemcpyHostToDevice));
                 else CK(cudaMemcpy(E.staging, ha->qu.data(), len * 2, cudaMemcpyHostToDevice));
+                CK(cudaStreamSynchronize(0));  // the copy's last part may still be on its way
                 g_uploaded += len * 2 + P.n_anodes[q] * 4;
                 k_to_dev<uint16_t><<<nb, kThreads, 0, E.stream>>>((const uint16_t*)E.staging, (uint16_t*)dst, E.xnodes[q], nh);
                 std::vector<float> sc(P.n_anodes[q]);
@@ -1117,6 +1119,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
                 src32 = img.data();
             }
             CK(cudaMemcpy(E.staging, src32, sp.tree.data_size[q] * 4, cudaMemcpyHostToDevice));
+            CK(cudaStreamSynchronize(0));
             g_uploaded += sp.tree.data_size[q] * 4;
             E.encode_staging(which, q);
             CK(cudaStreamSynchronize(E.stream));
@@ -1124,6 +1127,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     }
     E.upload_locks(host);
     if (leaf_net) E.leaf = std::make_unique<LeafEvaluator>(leaf_net, sp, P.leaves);
+    CK(cudaStreamSynchronize(0));  // zeroing and uploads, which the engine's stream does not wait for
     CK(cudaStreamSynchronize(E.stream));
     E.uploaded = g_uploaded;
 }

@@ -451,6 +451,10 @@ T* dnew(size_t n, bool zeroed = true) {
     if (zeroed) LCK(cudaMemset(p, 0, std::max<size_t>(n, 1) * sizeof(T)));
     return (T*)p;
 }
+// Zeroing and copies from pageable memory are queued on the legacy stream and
+// may still run when the call returns; the network's own streams do not wait
+// for that stream, so the host does, before they read or write what was filled.
+void settle() { LCK(cudaStreamSynchronize(cudaStreamLegacy)); }
 constexpr int kGatherSplit = 4;
 int pad128(int x) { return (x + 127) / 128 * 128; }
 int grid_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 16); }
@@ -504,6 +508,7 @@ double gemm_time_ms(int m, int n, int k, int reps) {
     unsigned* err = dnew<unsigned>(1);
     cudaStream_t s;
     cudaEvent_t e0, e1;
+    settle();
     LCK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     LCK(cudaEventCreate(&e0));
     LCK(cudaEventCreate(&e1));
@@ -591,6 +596,7 @@ LeafNet::LeafNet(const LeafNetDims& d, uint64_t seed) : d_(d) {
         LCK(cudaMemcpy(L->live, live.data(), nw, cudaMemcpyHostToDevice));
         L_.push_back(std::move(L));
     }
+    settle();
     for (int l = 0; l < layers(); l++) {
         Layer& L = *L_[l];
         const size_t nw = (size_t)L.out_p * L.in_p;
@@ -646,6 +652,7 @@ void LeafNet::ensure_rows(int rows_pad) {
         L.dzb = dnew<__nv_bfloat16>(n);
         L.dzt = dnew<__nv_bfloat16>(n);
     }
+    settle();
     rows_cap_ = rows_pad;
 }
 
@@ -757,6 +764,7 @@ void LeafNet::set_params(int l, const float* w, const float* b) {
     LCK(cudaStreamSynchronize(stream_));
     if (w) LCK(cudaMemcpy2D(L.w, L.in_p * 4, w, L.in * 4, L.in * 4, L.out, cudaMemcpyHostToDevice));
     if (b) LCK(cudaMemcpy(L.b, b, L.out * 4, cudaMemcpyHostToDevice));
+    settle();
     const size_t nw = (size_t)L.out_p * L.in_p;
     k_to_bf16<<<grid_for(nw), 256, 0, stream_>>>(L.w, nw, L.wb);
     k_transpose<<<dim3(L.in_p / 32, L.out_p / 32), dim3(32, 8), 0, stream_>>>(L.wb, L.out_p, L.in_p, L.wt);
@@ -774,7 +782,7 @@ namespace {
 template <class T>
 struct DevBuf {
     T* p = nullptr;
-    explicit DevBuf(size_t n, bool zeroed = true) : p(dnew<T>(n, zeroed)) {}
+    explicit DevBuf(size_t n) : p(dnew<T>(n, false)) {}
     ~DevBuf() { cudaFree(p); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -783,7 +791,7 @@ struct DevBuf {
 struct DevTable {
     DevBuf<float> buf;
     float* p;
-    DevTable(const float* h, size_t n) : buf(n, false), p(buf.p) {
+    DevTable(const float* h, size_t n) : buf(n), p(buf.p) {
         LCK(cudaMemcpy(p, h, n * 4, cudaMemcpyHostToDevice));
     }
 };
@@ -799,6 +807,7 @@ void LeafNet::forward_host(const float* x, int rows, float* y) {
     DevBuf<int> idx_buf(rows);
     int* didx = idx_buf.p;
     LCK(cudaMemcpy(didx, idx.data(), rows * 4, cudaMemcpyHostToDevice));
+    settle();
     k_gather_rows<<<dim3(rp, kGatherSplit), 256, 0, stream_>>>(X.p, nullptr, nullptr, didx, rows, d_.din, din_p_, d_.dout,
                                                                dout_p_, x_, nullptr, nullptr);
     forward(x_, rp, y_, false, stream_);
@@ -816,6 +825,7 @@ double LeafNet::gradients_host(const float* x, const float* t, const float* mask
     DevBuf<int> idx_buf(rows);
     int* didx = idx_buf.p;
     LCK(cudaMemcpy(didx, idx.data(), rows * 4, cudaMemcpyHostToDevice));
+    settle();
     k_gather_rows<<<dim3(rp, kGatherSplit), 256, 0, stream_>>>(X.p, T.p, M.p, didx, rows, d_.din, din_p_, d_.dout, dout_p_,
                                                                x_, t_, m_);
     forward(x_, rp, y_, true, stream_);
@@ -835,6 +845,7 @@ void LeafNet::train_host(const float* x, const float* t, const float* mask, int 
     const int nb = std::max(1, n / batch);  // whole batches (one short batch when n < batch)
     DevBuf<int> idx_buf(n);
     DevBuf<double> loss_buf(nb);  // a step's loss each, read at the epoch's end: the steps need no host in between
+    settle();
     std::vector<double> loss(nb);
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
@@ -1013,6 +1024,7 @@ LeafEvaluator::LeafEvaluator(std::shared_ptr<LeafNet> net, const Spot& sp, const
     mass_ = dnew<float>((size_t)rows_ * 2);
     err_ = dnew<float>((size_t)rows_);
     net_->reserve_rows(rows_p_);
+    settle();
 }
 
 LeafEvaluator::~LeafEvaluator() {

@@ -155,3 +155,22 @@ def test_one_adam_step():
             big = np.abs(gr) > 1e-5
             assert big.any() and np.abs(got - want)[big].max() <= 1e-2 * lr
             assert np.abs(got - w).max() <= lr * 1.001
+
+
+@pytest.mark.parametrize("rows,batch", [(200, 128), (300, 512)])
+def test_short_training_repeats(rows, batch):
+    """A call's tables are on the device before its first step reads them: the
+    same short training gives the same parameters every time, bit for bit
+    (buffers are zeroed and filled on a stream that the network's does not
+    wait for)."""
+    dims = (2705, 128, 1, 2652)
+    rng = np.random.default_rng(rows)
+    x, t = (rng.standard_normal((rows, w), np.float32) for w in (dims[0], dims[3]))
+    m = np.ones((rows, dims[3]), np.float32)
+    first = None
+    for _ in range(6):
+        net = g.LeafNet(*dims, seed=4)
+        net.train(x, t, m, epochs=2, batch=batch, lr=1e-3, seed=2)
+        got = [a for layer in range(dims[2] + 1) for a in net.params(layer)]
+        first = first or got
+        assert all(np.array_equal(a, b) for a, b in zip(first, got))
