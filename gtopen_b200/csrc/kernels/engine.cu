@@ -61,24 +61,28 @@ const char* const kKernelNames[7] = {"copy_root", "down_action", "down_chance", 
     } while (0)
 
 static thread_local uint64_t g_uploaded = 0;  // host-to-device bytes of the engine being built
+// Uploads and zeroing go on the stream whose kernels use the memory: the
+// engines' streams do not wait for the legacy stream, where a copy from
+// pageable memory or a fill may still run when its call returns.  (Pageable
+// memory is staged before cudaMemcpyAsync returns, so v may go.)
 template <class V>
-static typename V::value_type* dupload(const V& v, std::vector<void*>& owned, size_t* bytes) {
+static typename V::value_type* dupload(const V& v, std::vector<void*>& owned, size_t* bytes, cudaStream_t s) {
     using T = typename V::value_type;
     T* p = nullptr;
     const size_t n = std::max<size_t>(v.size(), 1);
     CK(cudaMalloc(&p, n * sizeof(T)));
     owned.push_back(p);
     *bytes += n * sizeof(T);
-    if (!v.empty()) CK(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (!v.empty()) CK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
     g_uploaded += v.size() * sizeof(T);
     return p;
 }
-static void* dalloc(size_t bytes, std::vector<void*>& owned, size_t* total) {
+static void* dalloc(size_t bytes, std::vector<void*>& owned, size_t* total, cudaStream_t s) {
     void* p = nullptr;
     CK(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
     owned.push_back(p);
     *total += bytes;
-    CK(cudaMemset(p, 0, std::max<size_t>(bytes, 16)));
+    CK(cudaMemsetAsync(p, 0, std::max<size_t>(bytes, 16), s));
     return p;
 }
 // A kernel's dynamic shared-memory limit is per function and process: raise it
@@ -265,10 +269,9 @@ struct EngineImpl {
         const size_t b0 = off[0].size() * 8, b1 = off[1].size() * 8, bs = sig.size() * 4;
         CK(cudaMalloc(&lock_buf, b0 + b1 + bs));
         char* base = (char*)lock_buf;
-        CK(cudaMemcpy(base, off[0].data(), b0, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(base + b0, off[1].data(), b1, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(base + b0 + b1, sig.data(), bs, cudaMemcpyHostToDevice));
-        CK(cudaStreamSynchronize(0));  // before the engine's own (non-blocking) stream reads them
+        CK(cudaMemcpyAsync(base, off[0].data(), b0, cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(base + b0, off[1].data(), b1, cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(base + b0 + b1, sig.data(), bs, cudaMemcpyHostToDevice, stream));
         d.lock_off[0] = (const long long*)base;
         d.lock_off[1] = (const long long*)(base + b0);
         d.lock_sig = (const float*)(base + b0 + b1);
@@ -703,8 +706,8 @@ static void setup_river(EngineImpl& E, const Spot& sp) {
     if (nslot < 2) return;  // the level sweeps keep the river
     auto& O = E.owned;
     size_t& B = E.bytes;
-    E.rtrees = dupload(P.rtrees, O, &B);
-    E.rsteps = dupload(P.rsteps, O, &B);
+    E.rtrees = dupload(P.rtrees, O, &B, E.stream);
+    E.rsteps = dupload(P.rsteps, O, &B, E.stream);
     E.ntrees = (int)P.rtrees.size();
     const uint32_t msort = P.max_sorted;
     for (int o = 0; o < 2; o++) {
@@ -735,8 +738,8 @@ static void setup_river(EngineImpl& E, const Spot& sp) {
             }
         }
         off.push_back((uint32_t)img.size());
-        E.d.rtab[o] = dupload(img, O, &B);
-        E.d.rtab_off[o] = dupload(off, O, &B);
+        E.d.rtab[o] = dupload(img, O, &B, E.stream);
+        E.d.rtab_off[o] = dupload(off, O, &B, E.stream);
     }
     river_smem_attrs<kDevF32>(need);
     river_smem_attrs<kDevI16>(need);
@@ -779,10 +782,9 @@ static void setup_shows(EngineImpl& E) {
     auto& O = E.owned;
     size_t& B = E.bytes;
     for (int q = 0; q < 2; q++) {
-        sg.ranks[q] = dalloc((size_t)P.num_slots * P.nh[q] * hand_rank_bytes(), O, &B);
-        sg.img[q] = dalloc((size_t)P.num_slots * show_image_bytes(sg.shape[q], sg.max_sorted[q]), O, &B);
+        sg.ranks[q] = dalloc((size_t)P.num_slots * P.nh[q] * hand_rank_bytes(), O, &B, E.stream);
+        sg.img[q] = dalloc((size_t)P.num_slots * show_image_bytes(sg.shape[q], sg.max_sorted[q]), O, &B, E.stream);
     }
-    CK(cudaStreamSynchronize(0));  // the tables' zeroing, before the engine's own (non-blocking) stream writes them
     build_show_tables(d, sg, P.num_slots, E.stream);
     CK(cudaGetLastError());
     auto group = [&](bool upper_only) {
@@ -809,7 +811,7 @@ static void setup_shows(EngineImpl& E) {
             std::copy(P.show.begin() + b.start, P.show.begin() + b.start + b.count, it.begin() + at[b.slot]);
             at[b.slot] += b.count;
         });
-        g.items = dupload(it, O, &B);
+        g.items = dupload(it, O, &B, E.stream);
         g.count = (uint32_t)(items / G);
         return g;
     };
@@ -904,48 +906,48 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     d.max_nterm = (int)max_nterm;
     for (int q = 0; q < 2; q++) {
         const Hands& h = sp.hands[q];
-        d.c1[q] = dupload(h.c1, O, &B);
-        d.c2[q] = dupload(h.c2, O, &B);
-        d.mask[q] = dupload(h.mask, O, &B);
-        d.same[q] = dupload(sp.same[q], O, &B);
-        d.w[q] = dupload(h.w, O, &B);
+        d.c1[q] = dupload(h.c1, O, &B, E.stream);
+        d.c2[q] = dupload(h.c2, O, &B, E.stream);
+        d.mask[q] = dupload(h.mask, O, &B, E.stream);
+        d.same[q] = dupload(sp.same[q], O, &B, E.stream);
+        d.w[q] = dupload(h.w, O, &B, E.stream);
         std::vector<uint16_t> hp;
         for (auto& t : sp.hand_perm[q]) hp.insert(hp.end(), t.begin(), t.end());
-        d.hperm[q] = dupload(hp, O, &B);
-        d.hcard_off[q] = dupload(P.hcard_off[q], O, &B);
-        d.hcard_idx[q] = dupload(P.hcard_idx[q], O, &B);
-        d.sorted_off[q] = dupload(P.sorted_off[q], O, &B);
-        d.sorted_cnt[q] = dupload(P.sorted_cnt[q], O, &B);
-        d.sorted_idx[q] = dupload(P.sorted_idx[q], O, &B);
-        d.ccard_off[q] = dupload(P.ccard_off[q], O, &B);
-        d.ccard_pos[q] = dupload(P.ccard_pos[q], O, &B);
-        d.ccard_card[q] = dupload(P.ccard_card[q], O, &B);
-        d.bin_off[q] = dupload(P.bin_off[q], O, &B);
-        d.bin_start[q] = dupload(P.bin_start[q], O, &B);
-        d.rank_off[q] = dupload(P.rank_off[q], O, &B);
-        d.rank_cnt[q] = dupload(P.rank_cnt[q], O, &B);
-        d.rank[q] = dupload(P.rank[q], O, &B);
-        d.zero_off[q] = dupload(P.zero_off[q], O, &B);
-        d.zero_idx[q] = dupload(P.zero_idx[q], O, &B);
-        d.reach[q] = (float*)dalloc(P.n_rslots[q] * (size_t)d.rstr[q] * sizeof(float), O, &B);
-        d.node_id[q] = dupload(P.anode_id[q], O, &B);
+        d.hperm[q] = dupload(hp, O, &B, E.stream);
+        d.hcard_off[q] = dupload(P.hcard_off[q], O, &B, E.stream);
+        d.hcard_idx[q] = dupload(P.hcard_idx[q], O, &B, E.stream);
+        d.sorted_off[q] = dupload(P.sorted_off[q], O, &B, E.stream);
+        d.sorted_cnt[q] = dupload(P.sorted_cnt[q], O, &B, E.stream);
+        d.sorted_idx[q] = dupload(P.sorted_idx[q], O, &B, E.stream);
+        d.ccard_off[q] = dupload(P.ccard_off[q], O, &B, E.stream);
+        d.ccard_pos[q] = dupload(P.ccard_pos[q], O, &B, E.stream);
+        d.ccard_card[q] = dupload(P.ccard_card[q], O, &B, E.stream);
+        d.bin_off[q] = dupload(P.bin_off[q], O, &B, E.stream);
+        d.bin_start[q] = dupload(P.bin_start[q], O, &B, E.stream);
+        d.rank_off[q] = dupload(P.rank_off[q], O, &B, E.stream);
+        d.rank_cnt[q] = dupload(P.rank_cnt[q], O, &B, E.stream);
+        d.rank[q] = dupload(P.rank[q], O, &B, E.stream);
+        d.zero_off[q] = dupload(P.zero_off[q], O, &B, E.stream);
+        d.zero_idx[q] = dupload(P.zero_idx[q], O, &B, E.stream);
+        d.reach[q] = (float*)dalloc(P.n_rslots[q] * (size_t)d.rstr[q] * sizeof(float), O, &B, E.stream);
+        d.node_id[q] = dupload(P.anode_id[q], O, &B, E.stream);
     }
-    d.cards = dupload(P.cards, O, &B);
+    d.cards = dupload(P.cards, O, &B, E.stream);
     if (!E.vec) {  // the vector kernels' node records hold all of it
-        d.crefs = dupload(P.crefs, O, &B);
-        d.terms = dupload(P.terms, O, &B);
+        d.crefs = dupload(P.crefs, O, &B, E.stream);
+        d.terms = dupload(P.terms, O, &B, E.stream);
     }
-    d.cfv = (float*)dalloc(P.n_cslots * (size_t)d.nh_max * sizeof(float), O, &B);
-    d.disc = (float*)dalloc(4 * sizeof(float), O, &B);
-    d.iter = (unsigned*)dalloc(sizeof(unsigned), O, &B);
-    d.dot = (double*)dalloc(4 * sizeof(double), O, &B);
-    d.err = (unsigned*)dalloc(sizeof(unsigned), O, &B);
-    CK(cudaMemcpy(d.iter, &E.iteration, sizeof(unsigned), cudaMemcpyHostToDevice));
-    if (!E.vec) E.act = dupload(P.act, O, &B);
-    E.edge = dupload(P.edge, O, &B);
-    E.fold = dupload(P.fold, O, &B);
-    if (!E.vec) E.show = dupload(P.show, O, &B);
-    E.chance = dupload(P.chance, O, &B);
+    d.cfv = (float*)dalloc(P.n_cslots * (size_t)d.nh_max * sizeof(float), O, &B, E.stream);
+    d.disc = (float*)dalloc(4 * sizeof(float), O, &B, E.stream);
+    d.iter = (unsigned*)dalloc(sizeof(unsigned), O, &B, E.stream);
+    d.dot = (double*)dalloc(4 * sizeof(double), O, &B, E.stream);
+    d.err = (unsigned*)dalloc(sizeof(unsigned), O, &B, E.stream);
+    CK(cudaMemcpyAsync(d.iter, &E.iteration, sizeof(unsigned), cudaMemcpyHostToDevice, E.stream));
+    if (!E.vec) E.act = dupload(P.act, O, &B, E.stream);
+    E.edge = dupload(P.edge, O, &B, E.stream);
+    E.fold = dupload(P.fold, O, &B, E.stream);
+    if (!E.vec) E.show = dupload(P.show, O, &B, E.stream);
+    E.chance = dupload(P.chance, O, &B, E.stream);
     const size_t tsz = E.term64 ? sizeof(double) : sizeof(float);
     E.show_smem = (size_t)d.scr_elems * sizeof(double);
     if (E.warp) E.warp_smem = (size_t)kWarps * d.nh_pad * sizeof(float);
@@ -976,13 +978,13 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
         });
         E.nfolds = (uint32_t)fs[0].size();
         for (int q = 0; q < 2; q++) {
-            E.fold_slots[q] = dupload(fs[q], O, &B);
+            E.fold_slots[q] = dupload(fs[q], O, &B, E.stream);
             size_t fsm;
             const void* fn[2];
             fold_kernels(P.nh[q], fn, &fsm);
             for (const void* f : fn) set_smem(f, fsm);
         }
-        d.folds = (const FoldSum*)dalloc((size_t)E.nfolds * fold_sum_bytes(), O, &B);
+        d.folds = (const FoldSum*)dalloc((size_t)E.nfolds * fold_sum_bytes(), O, &B, E.stream);
         auto records = [&](auto KA) {
             constexpr int K = KA();
             PodVec<SNodeT<K>> sn(P.act.size());
@@ -1017,7 +1019,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
                     }
                 }
             });
-            return dupload(sn, O, &B);
+            return dupload(sn, O, &B, E.stream);
         };
         if (E.staged) E.snodes = records(std::integral_constant<int, kSKA>{});
         else E.wnodes = records(std::integral_constant<int, kVKA>{});
@@ -1028,7 +1030,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
                 const uint32_t s = sp.same[q][i];
                 hi[i] = (uint32_t)h.c1[i] | (uint32_t)h.c2[i] << 6 | (s == kSentinel ? 0xFFFFu : s) << 16;
             }
-            d.hinfo[q] = dupload(hi, O, &B);
+            d.hinfo[q] = dupload(hi, O, &B, E.stream);
         }
     }
     if (E.staged) {
@@ -1062,22 +1064,22 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     const size_t esz = (size_t)fmt_bytes(E.fmt);
     for (int q = 0; q < 2; q++) {
         const size_t len = P.arena_len[q];
-        E.ar.reg[q] = dalloc(len * esz, O, &B);
-        E.ar.str[q] = dalloc(len * esz, O, &B);
-        E.ar.pred[q] = E.pcfr ? dalloc(len * esz, O, &B) : nullptr;
+        E.ar.reg[q] = dalloc(len * esz, O, &B, E.stream);
+        E.ar.str[q] = dalloc(len * esz, O, &B, E.stream);
+        E.ar.pred[q] = E.pcfr ? dalloc(len * esz, O, &B, E.stream) : nullptr;
         if (E.fmt != kFmtF32) {
-            E.ar.rscale[q] = (float*)dalloc(std::max<uint64_t>(P.n_anodes[q], 1) * 4, O, &B);
-            E.ar.sscale[q] = (float*)dalloc(std::max<uint64_t>(P.n_anodes[q], 1) * 4, O, &B);
-            E.ar.pscale[q] = E.pcfr ? (float*)dalloc(std::max<uint64_t>(P.n_anodes[q], 1) * 4, O, &B) : nullptr;
+            E.ar.rscale[q] = (float*)dalloc(std::max<uint64_t>(P.n_anodes[q], 1) * 4, O, &B, E.stream);
+            E.ar.sscale[q] = (float*)dalloc(std::max<uint64_t>(P.n_anodes[q], 1) * 4, O, &B, E.stream);
+            E.ar.pscale[q] = E.pcfr ? (float*)dalloc(std::max<uint64_t>(P.n_anodes[q], 1) * 4, O, &B, E.stream) : nullptr;
         }
         for (uint64_t s = 0; s < P.n_anodes[q]; s++) {
             const uint32_t nd = P.anode_id[q][s];
             E.hx[q].push_back({sp.tree.data_off[nd], P.anode_off[q][s], sp.tree.nchild[nd], (uint32_t)s});
         }
-        E.xnodes[q] = dupload(E.hx[q], O, &B);
+        E.xnodes[q] = dupload(E.hx[q], O, &B, E.stream);
     }
     E.staging_len = std::max<uint64_t>(std::max(sp.tree.data_size[0], sp.tree.data_size[1]), 1);
-    E.staging = (float*)dalloc(E.staging_len * sizeof(float), O, &B);
+    E.staging = (float*)dalloc(E.staging_len * sizeof(float), O, &B, E.stream);
     // read-back chunks only where an arena is worth them (pinning takes a few ms)
     const bool big = E.staging_len * sizeof(float) >= 2 * kPinChunk;
     CK(cudaMallocHost(&E.h_dot, 4096 + (big ? 2 * kPinChunk : 0)));
@@ -1098,9 +1100,8 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
             if (!ha) continue;  // predictions start at zero
             if (E.fmt == kFmtI16 && ha->kind != 0) {
                 const size_t len = sp.tree.data_size[q];
-                if (ha->kind == 1) CK(cudaMemcpy(E.staging, ha->qi.data(), len * 2, cudaMemcpyHostToDevice));
-                else CK(cudaMemcpy(E.staging, ha->qu.data(), len * 2, cudaMemcpyHostToDevice));
-                CK(cudaStreamSynchronize(0));  // the copy's last part may still be on its way
+                if (ha->kind == 1) CK(cudaMemcpyAsync(E.staging, ha->qi.data(), len * 2, cudaMemcpyHostToDevice, E.stream));
+                else CK(cudaMemcpyAsync(E.staging, ha->qu.data(), len * 2, cudaMemcpyHostToDevice, E.stream));
                 g_uploaded += len * 2 + P.n_anodes[q] * 4;
                 k_to_dev<uint16_t><<<nb, kThreads, 0, E.stream>>>((const uint16_t*)E.staging, (uint16_t*)dst, E.xnodes[q], nh);
                 std::vector<float> sc(P.n_anodes[q]);
@@ -1118,8 +1119,7 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
                 host.arena_f32(which, q, img.data());
                 src32 = img.data();
             }
-            CK(cudaMemcpy(E.staging, src32, sp.tree.data_size[q] * 4, cudaMemcpyHostToDevice));
-            CK(cudaStreamSynchronize(0));
+            CK(cudaMemcpyAsync(E.staging, src32, sp.tree.data_size[q] * 4, cudaMemcpyHostToDevice, E.stream));
             g_uploaded += sp.tree.data_size[q] * 4;
             E.encode_staging(which, q);
             CK(cudaStreamSynchronize(E.stream));
@@ -1127,7 +1127,6 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     }
     E.upload_locks(host);
     if (leaf_net) E.leaf = std::make_unique<LeafEvaluator>(leaf_net, sp, P.leaves);
-    CK(cudaStreamSynchronize(0));  // zeroing and uploads, which the engine's stream does not wait for
     CK(cudaStreamSynchronize(E.stream));
     E.uploaded = g_uploaded;
 }
@@ -1244,7 +1243,7 @@ void GpuEngine::export_arena(int which, int p, float* out) {
                 x.host_off = at;
                 at += (uint64_t)x.na * nh;
             }
-            E.xpacked[p] = dupload(xs, E.owned, &E.bytes);
+            E.xpacked[p] = dupload(xs, E.owned, &E.bytes, E.stream);
         }
         decode_blocks(which, p, E.xpacked[p]);
         std::vector<float> tmp(held);
@@ -1909,8 +1908,8 @@ struct BatchImpl {
         for (size_t s = 0; s < E.size(); s++) {
             EngineImpl& X = *E[s];
             if (!X.show) {  // the level-ordered showdowns: the batched kernel's only
-                X.show = dupload(X.plan.show, X.owned, &X.bytes);
-                X.show_batch = dupload(X.plan.show_batch, X.owned, &X.bytes);
+                X.show = dupload(X.plan.show, X.owned, &X.bytes, stream);
+                X.show_batch = dupload(X.plan.show_batch, X.owned, &X.bytes, stream);
             }
             BSpot& b = hs[s];
             std::memset(&b, 0, sizeof(b));
@@ -1946,10 +1945,10 @@ struct BatchImpl {
         if (t >= 0xFFFFFFFFull) throw Error("batch: too many tickets in one iteration");
         nticket = (unsigned)t;
         nseg = (int)hg.size();
-        spots = dupload(hs, owned, &bytes);
-        segs = dupload(hg, owned, &bytes);
+        spots = dupload(hs, owned, &bytes, stream);
+        segs = dupload(hg, owned, &bytes, stream);
         nctl = (size_t)kBCtlDone + E.size();
-        ctl = (unsigned*)dalloc(nctl * sizeof(unsigned), owned, &bytes);
+        ctl = (unsigned*)dalloc(nctl * sizeof(unsigned), owned, &bytes, stream);
         set_smem(kernel_fn(), smem);
         int dev = 0, nsm = 0;
         CK(cudaGetDevice(&dev));
