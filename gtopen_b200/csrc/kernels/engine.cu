@@ -1907,10 +1907,11 @@ struct BatchImpl {
         std::vector<const Plan*> plans;
         for (size_t s = 0; s < E.size(); s++) {
             EngineImpl& X = *E[s];
-            if (!X.show) {  // the level-ordered showdowns: the batched kernel's only
-                X.show = dupload(X.plan.show, X.owned, &X.bytes, stream);
-                X.show_batch = dupload(X.plan.show_batch, X.owned, &X.bytes, stream);
-            }
+            // the level-ordered showdowns: the batched kernel's only.  On the
+            // engine's stream, which ready() waits for, whatever batch asks;
+            // each by itself, so that a failed upload is made up for later
+            if (!X.show) X.show = dupload(X.plan.show, X.owned, &X.bytes, X.stream);
+            if (!X.show_batch) X.show_batch = dupload(X.plan.show_batch, X.owned, &X.bytes, X.stream);
             BSpot& b = hs[s];
             std::memset(&b, 0, sizeof(b));
             b.d = X.d;
