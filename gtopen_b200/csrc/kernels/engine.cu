@@ -879,6 +879,9 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     E.wide = P.max_children > 8u;
     E.staged = staged_kind && P.max_children <= (uint32_t)kSKA;
     E.vec = staged_kind && P.max_children <= (uint32_t)kVKA;
+    if (E.vec)  // its sweeps evaluate every fold in its parent and launch no other fold kernel
+        for (const Span& s : P.fold_span)
+            if (s.count) throw Error("internal: a fold terminal with a slot of its own in a plan of in-place folds");
     if (E.fmt == kFmtFP8 && !E.staged) throw Error("FP8 arenas need nodes of at most 4 actions (the staged kernels)");
     if (P.nh_max > kThreads * kMaxHpt) throw Error("more than 1536 hands per player is not supported on the GPU");
     CK(cudaStreamCreateWithFlags(&E.stream, cudaStreamNonBlocking));
