@@ -175,6 +175,7 @@ def lib():
         "gtob_net_forward": (I, [P, P, I, P]),
         "gtob_net_gradients": (I, [P, P, P, P, I, C.POINTER(D)]),
         "gtob_net_train": (I, [P, P, P, P, I, I, I, C.c_float, U64, P]),
+        "gtob_net_inject_error": (I, [P]),
         "gtob_gemm_bf16": (I, [P, P, I, I, I, P]),
         "gtob_gpu_new_dl": (I, [P, P, I, I, C.POINTER(P)]),
         "gtob_gpu_leaves": (I, [P, P, P, P, I, C.POINTER(I)]),
@@ -964,6 +965,10 @@ class LeafNet:
         _check(lib().gtob_net_train(self._h, _ptr(x), _ptr(t), _ptr(m), x.shape[0], int(epochs), int(batch),
                                     C.c_float(lr), int(seed), _ptr(losses)))
         return losses
+
+    def inject_error(self):
+        """Tests: the device error word as a product whose wait gave up leaves it."""
+        _check(lib().gtob_net_inject_error(self._h))
 
 
 def dl_gpu_solver(solver, net, device_format=None, engine="staged"):

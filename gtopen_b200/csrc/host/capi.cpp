@@ -777,6 +777,12 @@ int gtob_net_train(gtob_net* n, const float* x, const float* t, const float* mas
     n->n->train_host(x, t, mask, count, epochs, batch, lr, seed, losses);
     API_END
 }
+int gtob_net_inject_error(gtob_net* n) {
+    REQUIRE(n);
+    API_BEGIN
+    n->n->inject_error();
+    API_END
+}
 int gtob_gpu_new_dl(const gtob_solver* v, gtob_net* net, int fmt, int engine, gtob_gpu** out) {
     REQUIRE(v && net && out && fmt >= -1 && fmt <= 3 && engine >= GTOB_ENGINE_FUSED && engine <= GTOB_ENGINE_STAGED_RIVER);
     *out = nullptr;

@@ -80,11 +80,14 @@ __device__ __forceinline__ bool bar_try(uint64_t* b, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __noinline__ bool bar_wait(uint64_t* b, unsigned parity) {
+// err: an earlier product's failure ends the wait at once (the products queued
+// behind it would run out their limit one by one); null: the full limit, for
+// what has to finish before a CTA may leave.
+__device__ __noinline__ bool bar_wait(uint64_t* b, unsigned parity, const volatile unsigned* err) {
     if (bar_try(b, parity)) return true;
     const unsigned long long t0 = gtimer();
     while (!bar_try(b, parity))
-        if (gtimer() - t0 > kNetWaitNs) return false;
+        if (gtimer() - t0 > kNetWaitNs || (err && *err)) return false;
     return true;
 }
 __device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         int kb = 0;
         for (; kb < nk; kb++) {
             const int s = kb % kStages;
-            if (kb >= kStages && !bar_wait(&empty[s], ((kb / kStages) & 1) ^ 1)) {
+            if (kb >= kStages && !bar_wait(&empty[s], ((kb / kStages) & 1) ^ 1, err)) {
                 atomicOr(err, kErrGemmWait);
                 aborted = 1;
                 break;
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     } else if (warp == 1 && lane == 0) {  // MMA issuer
         for (int kb = 0; kb < nk; kb++) {
             const int s = kb % kStages;
-            if (!bar_wait(&full[s], (kb / kStages) & 1)) {
+            if (!bar_wait(&full[s], (kb / kStages) & 1, err)) {
                 atomicOr(err, kErrGemmWait);
                 aborted = 1;
                 break;
@@ -247,7 +250,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         tm_commit(&done);  // arrives when every product issued above has finished
     }
     __syncwarp();
-    const bool ok = bar_wait(&done, 0);
+    const bool ok = bar_wait(&done, 0, err);
     const int good = __syncthreads_and(ok ? 1 : 0) && !aborted;
     if (!ok && threadIdx.x == 0) atomicOr(err, kErrGemmWait);
     if (!good) {
@@ -258,10 +261,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // producer, for the tile loads it issued that no product waited
         // for (at most the last kStages: a load is only issued once the
         // product kStages before it has read its stage).
-        if (!ok) bar_wait(&done, 0);
+        if (!ok) bar_wait(&done, 0, nullptr);
         if (warp == 0 && lane == 0)
             for (int kb = issued > kStages ? issued - kStages : 0; kb < issued; kb++)
-                bar_wait(&full[kb % kStages], (kb / kStages) & 1);
+                bar_wait(&full[kb % kStages], (kb / kStages) & 1, nullptr);
     }
     tm_fence_after();
     if (good) {
@@ -355,6 +358,8 @@ __global__ void __launch_bounds__(256) k_colsum(const float* __restrict__ g, int
 // (masters, moments, the bf16 copy and its transpose, which the next step's
 // products read), then the biases; padded weights (live = 0) stay zero.
 // 8.4M parameters: twelve launches, 120 us -> one, bound by HBM.
+// A step whose products gave up (err) changes nothing: the host reads err once
+// an epoch, and weights and moments stay those of the last whole step (applied).
 struct AdamLayer {
     float *w, *g, *m, *v, *b, *gb, *mb, *vb;
     const uint8_t* live;
@@ -377,9 +382,12 @@ __device__ __forceinline__ float adam_one(float& w, float g, float& m, float& v,
     return w;
 }
 __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamLayers A, float lr, float b1, float b2,
-                                              float eps, float bc1, float bc2) {
+                                              float eps, float bc1, float bc2, const unsigned* err, int step,
+                                              int* applied) {
     __shared__ __nv_bfloat16 t[32][33];
     const int blk = (int)blockIdx.x, c = threadIdx.x & 31, r0 = threadIdx.x >> 5;
+    if (*err) return;
+    if (blk == 0 && threadIdx.x == 0) *applied = step;
     for (int k = 0; k < A.n; k++) {
         const AdamLayer& L = A.l[k];
         const int tiles = (L.in_p / 32) * (L.out_p / 32);
@@ -567,6 +575,7 @@ LeafNet::LeafNet(const LeafNetDims& d, uint64_t seed) : d_(d) {
     LCK(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming));
     err_ = dnew<unsigned>(1);
     loss_ = dnew<double>(1);
+    applied_ = dnew<int>(1);
     uint64_t s = seed * 0x9E3779B97F4A7C15ull + 0x2545F4914F6CDD1Dull;
     if (!s) s = 1;
     for (int l = 0; l <= d.nhidden; l++) {
@@ -610,7 +619,7 @@ LeafNet::~LeafNet() {
     if (stream_) cudaStreamSynchronize(stream_);
     L_.clear();
     for (void* p : {(void*)x_, (void*)xt_, (void*)dyb_, (void*)dyt_, (void*)y_, (void*)dy_, (void*)t_, (void*)m_,
-                    (void*)loss_, (void*)err_})
+                    (void*)loss_, (void*)err_, (void*)applied_})
         cudaFree(p);
     if (ev_) cudaEventDestroy(ev_);
     if (side_) cudaStreamDestroy(side_);
@@ -622,9 +631,16 @@ void LeafNet::check(cudaStream_t s) {
     unsigned e = 0;
     LCK(cudaMemcpy(&e, err_, sizeof(e), cudaMemcpyDeviceToHost));
     if (e) {
-        LCK(cudaMemset(err_, 0, sizeof(unsigned)));
+        LCK(cudaMemsetAsync(err_, 0, sizeof(unsigned), s));
+        LCK(cudaStreamSynchronize(s));
         throw Error("timeout: a tensor-core matrix product's wait gave up");
     }
+}
+
+void LeafNet::inject_error() {
+    LCK(cudaStreamSynchronize(stream_));
+    LCK(cudaMemsetAsync(err_, 0xFF, sizeof(unsigned), stream_));
+    LCK(cudaStreamSynchronize(stream_));
 }
 
 void LeafNet::ensure_rows(int rows_pad) {
@@ -739,7 +755,7 @@ void LeafNet::adam(float lr, int step, cudaStream_t s) {
         a.bias0 = blocks;
         blocks += (L.out + 255) / 256;
     }
-    k_adam<<<blocks, 256, 0, s>>>(A, lr, b1, b2, eps, bc1, bc2);
+    k_adam<<<blocks, 256, 0, s>>>(A, lr, b1, b2, eps, bc1, bc2, err_, step, applied_);
     launches_++;
     LCK(cudaGetLastError());
 }
@@ -864,7 +880,12 @@ void LeafNet::train_host(const float* x, const float* t, const float* mask, int 
             adam(lr, ++adam_t_, stream_);
         }
         LCK(cudaMemcpyAsync(loss.data(), loss_buf.p, (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-        check(stream_);
+        try {
+            check(stream_);
+        } catch (...) {  // the epoch's steps from the failed one on were not applied
+            cudaMemcpy(&adam_t_, applied_, sizeof(int), cudaMemcpyDeviceToHost);
+            throw;
+        }
         double sum = 0.0;
         for (double x : loss) sum += x;
         if (losses) losses[ep] = (float)(sum / std::max(nb, 1));

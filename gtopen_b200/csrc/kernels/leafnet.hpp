@@ -59,7 +59,9 @@ class LeafNet {
     // one forward + backward over rows samples (masked mean squared error);
     // gradients stay on the device (get_grads); returns the loss
     double gradients_host(const float* x, const float* t, const float* mask, int rows);
-    // epochs of Adam over n samples in shuffled batches; per-epoch mean loss
+    // epochs of Adam over n samples in shuffled batches; per-epoch mean loss.
+    // On an error the parameters are those after the last step whose products
+    // all finished
     void train_host(const float* x, const float* t, const float* mask, int n, int epochs, int batch, float lr,
                     uint64_t seed, float* losses);
     // device buffers for rows_pad rows: call before capturing forward_device
@@ -71,6 +73,8 @@ class LeafNet {
     int dout_pad() const { return dout_p_; }
     unsigned* err_word() const { return err_; }
     uint32_t kernel_launches() const { return launches_; }
+    // tests: the error word as a product whose wait gave up leaves it
+    void inject_error();
 
   private:
     struct Layer;
@@ -88,7 +92,8 @@ class LeafNet {
     float *y_ = nullptr, *dy_ = nullptr, *t_ = nullptr, *m_ = nullptr;
     double* loss_ = nullptr;
     unsigned* err_ = nullptr;
-    int adam_t_ = 0;
+    int adam_t_ = 0;          // Adam steps taken,
+    int* applied_ = nullptr;  // and the last one the device applied
     uint32_t launches_ = 0;
     cudaStream_t stream_ = nullptr, side_ = nullptr;  // side_: weight gradients of a backward pass
     cudaEvent_t ev_ = nullptr;

@@ -447,9 +447,13 @@ int gtob_net_forward(gtob_net* net, const float* x, int rows, float* y);
 /* one forward + backward; *loss = the masked mean squared error */
 int gtob_net_gradients(gtob_net* net, const float* x, const float* t, const float* mask, int rows, double* loss);
 /* epochs of shuffled batches (batch a multiple of 128); losses[epoch] = the
- * epoch's mean batch loss (NULL: not reported) */
+ * epoch's mean batch loss (NULL: not reported).  A product whose bounded wait
+ * gives up ends the call with an error at its epoch's end; the parameters are
+ * then those after the last step whose products all finished. */
 int gtob_net_train(gtob_net* net, const float* x, const float* t, const float* mask, int n, int epochs, int batch,
                    float lr, uint64_t seed, float* losses);
+/* tests: leaves the net's device error word as a product whose wait gave up does */
+int gtob_net_inject_error(gtob_net* net);
 /* A depth-limited flop solve: the plan cuts the tree at the chance nodes
  * dealing the turn where betting follows (all-in runouts stay exact), and
  * after every down sweep the net evaluates each such leaf for every turn

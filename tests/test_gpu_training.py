@@ -86,3 +86,25 @@ def test_training_follows_64_bits(n, batch, epochs):
         for a, e, b in zip(params, exact[k].ps, start[k]):
             e = e.detach().cpu().numpy()
             assert np.linalg.norm(a - e) <= 2.0 ** -5 * np.linalg.norm(e - b)
+
+
+def test_a_failed_product_leaves_the_last_good_step():
+    """A product whose wait gave up: the call ends with an error, and weights,
+    moments and step count are those of the last whole step -- the training
+    goes on as if the failed call had not been made."""
+    dims, n = (70, 130, 2, 40), 256
+    rng = np.random.default_rng(8)
+    x, t = rng.normal(0, 1, (n, 70)).astype(np.float32), rng.normal(0, 1, (n, 40)).astype(np.float32)
+    m = np.ones((n, 40), np.float32)
+    a, b = g.LeafNet(*dims, seed=3), g.LeafNet(*dims, seed=3)
+    params = lambda net: [p for layer in range(dims[2] + 1) for p in net.params(layer)]  # noqa: E731
+    for net in (a, b):
+        net.train(x, t, m, epochs=2, batch=128, lr=1e-2, seed=1)
+    before = params(a)
+    a.inject_error()
+    with pytest.raises(g.GtobError, match="timeout"):
+        a.train(x, t, m, epochs=2, batch=128, lr=1e-2, seed=2)
+    assert all(np.array_equal(p, q) for p, q in zip(before, params(a)))
+    for net in (a, b):
+        net.train(x, t, m, epochs=2, batch=128, lr=1e-2, seed=3)
+    assert all(np.array_equal(p, q) for p, q in zip(params(a), params(b)))
