@@ -69,7 +69,8 @@ class GpuEngine {
     // A depth-limited solve of a flop spot: the tree is cut at the chance
     // nodes dealing the turn (where betting follows) and their values come
     // from leaf_net after every down sweep.  The net serves one engine at a
-    // time (its activation buffers are its own).
+    // time (it has one error word, and its weights must not change while
+    // iterations are in flight); it may be trained between iterations.
     GpuEngine(const HostSolver& host, int fmt, int engine, std::shared_ptr<LeafNet> leaf_net)
         : GpuEngine(host, fmt, engine, 0, 1, nullptr, std::move(leaf_net)) {}
     bool fused() const;

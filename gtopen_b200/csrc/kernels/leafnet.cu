@@ -672,10 +672,12 @@ void LeafNet::ensure_rows(int rows_pad) {
     rows_cap_ = rows_pad;
 }
 
-void LeafNet::forward(const __nv_bfloat16* x, int rows_pad, float* y, bool keep, cudaStream_t s) {
+void LeafNet::forward(const __nv_bfloat16* x, int rows_pad, float* y, bool keep, __nv_bfloat16* const* h,
+                      cudaStream_t s) {
     const __nv_bfloat16* in = x;
     for (int l = 0; l < d_.nhidden; l++) {
         Layer& L = *L_[l];
+        __nv_bfloat16* out = h ? h[l & 1] : L.h;
         GemmEpilogue e;
         e.bias = L.b;
         if (keep) {
@@ -683,11 +685,11 @@ void LeafNet::forward(const __nv_bfloat16* x, int rows_pad, float* y, bool keep,
             e.ld_pre = L.out_p;
         }
         e.gelu = true;
-        e.out_bf16 = L.h;
+        e.out_bf16 = out;
         e.ld_bf16 = L.out_p;
         gemm_bf16_tn(in, L.wb, rows_pad, L.out_p, L.in_p, e, err_, s);
         launches_++;
-        in = L.h;
+        in = out;
     }
     Layer& O = *L_[d_.nhidden];
     GemmEpilogue e;
@@ -787,10 +789,10 @@ void LeafNet::set_params(int l, const float* w, const float* b) {
     check(stream_);
 }
 
-void LeafNet::forward_device(const __nv_bfloat16* x, int rows_pad, float* y, cudaStream_t s) {
+void LeafNet::forward_device(const __nv_bfloat16* x, int rows_pad, float* y, __nv_bfloat16* const (&h)[2],
+                             cudaStream_t s) {
     if (rows_pad % 128) throw Error("invalid argument: rows not padded to 128");
-    ensure_rows(rows_pad);
-    forward(x, rows_pad, y, false, s);
+    forward(x, rows_pad, y, false, h, s);
 }
 
 namespace {
@@ -826,7 +828,7 @@ void LeafNet::forward_host(const float* x, int rows, float* y) {
     settle();
     k_gather_rows<<<dim3(rp, kGatherSplit), 256, 0, stream_>>>(X.p, nullptr, nullptr, didx, rows, d_.din, din_p_, d_.dout,
                                                                dout_p_, x_, nullptr, nullptr);
-    forward(x_, rp, y_, false, stream_);
+    forward(x_, rp, y_, false, nullptr, stream_);
     check(stream_);
     LCK(cudaMemcpy2D(y, d_.dout * 4, y_, dout_p_ * 4, d_.dout * 4, rows, cudaMemcpyDeviceToHost));
 }
@@ -844,7 +846,7 @@ double LeafNet::gradients_host(const float* x, const float* t, const float* mask
     settle();
     k_gather_rows<<<dim3(rp, kGatherSplit), 256, 0, stream_>>>(X.p, T.p, M.p, didx, rows, d_.din, din_p_, d_.dout, dout_p_,
                                                                x_, t_, m_);
-    forward(x_, rp, y_, true, stream_);
+    forward(x_, rp, y_, true, nullptr, stream_);
     LCK(cudaMemsetAsync(loss_, 0, sizeof(double), stream_));
     backward(t_, m_, rp, rows, loss_, stream_);
     double loss = 0.0;
@@ -875,7 +877,7 @@ void LeafNet::train_host(const float* x, const float* t, const float* mask, int 
             const int b0 = bi * batch, rows = std::min(batch, n - b0);
             k_gather_rows<<<dim3(batch, kGatherSplit), 256, 0, stream_>>>(X.p, T.p, M.p, idx_buf.p + b0, rows, d_.din, din_p_,
                                                                           d_.dout, dout_p_, x_, t_, m_);
-            forward(x_, batch, y_, true, stream_);
+            forward(x_, batch, y_, true, nullptr, stream_);
             backward(t_, m_, batch, rows, loss_buf.p + bi, stream_);
             adam(lr, ++adam_t_, stream_);
         }
@@ -1044,14 +1046,14 @@ LeafEvaluator::LeafEvaluator(std::shared_ptr<LeafNet> net, const Spot& sp, const
     y_ = dnew<float>((size_t)rows_p_ * net_->dout_pad());
     mass_ = dnew<float>((size_t)rows_ * 2);
     err_ = dnew<float>((size_t)rows_);
-    net_->reserve_rows(rows_p_);
+    for (auto& h : h_) h = dnew<__nv_bfloat16>((size_t)rows_p_ * net_->hidden_pad());
     settle();
 }
 
 LeafEvaluator::~LeafEvaluator() {
     for (void* p : {(void*)leaves_, (void*)cards_, (void*)hmask_[0], (void*)hmask_[1], (void*)combo_[0],
-                    (void*)combo_[1], (void*)hand_of_[0], (void*)hand_of_[1], (void*)x_, (void*)y_, (void*)mass_,
-                    (void*)err_})
+                    (void*)combo_[1], (void*)hand_of_[0], (void*)hand_of_[1], (void*)x_, (void*)h_[0], (void*)h_[1],
+                    (void*)y_, (void*)mass_, (void*)err_})
         cudaFree(p);
 }
 
@@ -1079,7 +1081,7 @@ void LeafEvaluator::run(int p, const float* reach0, size_t rstr0, const float* r
     L.mass = mass_;
     L.err = err_;
     k_leaf_gather<<<rows_, 256, 0, s>>>(L);
-    net_->forward_device(x_, rows_p_, y_, s);
+    net_->forward_device(x_, rows_p_, y_, h_, s);
     k_leaf_err<<<rows_, 256, 0, s>>>(L);
     const int chunks = (nh_[p] + kScatterHands - 1) / kScatterHands;
     k_leaf_scatter<<<nleaves_ * chunks, kScatterHands * kScatterParts, 0, s>>>(L, p, cfv, cfv_stride, chunks);

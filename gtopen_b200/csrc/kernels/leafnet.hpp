@@ -64,11 +64,13 @@ class LeafNet {
     // all finished
     void train_host(const float* x, const float* t, const float* mask, int n, int epochs, int batch, float lr,
                     uint64_t seed, float* losses);
-    // device buffers for rows_pad rows: call before capturing forward_device
-    void reserve_rows(int rows_pad) { ensure_rows(rows_pad); }
     // device-side forward over rows padded inputs (bf16, rows_pad x din_pad,
-    // rows_pad a multiple of 128) into f32 outputs (rows_pad x dout_pad)
-    void forward_device(const __nv_bfloat16* x, int rows_pad, float* y, cudaStream_t s);
+    // rows_pad a multiple of 128) into f32 outputs (rows_pad x dout_pad).  h:
+    // the caller's activations, rows_pad x hidden_pad each, taken by the layers
+    // in turn -- a captured pass must not point at the network's own buffers,
+    // which grow (and move) with the largest batch it is trained on
+    void forward_device(const __nv_bfloat16* x, int rows_pad, float* y, __nv_bfloat16* const (&h)[2], cudaStream_t s);
+    int hidden_pad() const { return dh_p_; }
     int din_pad() const { return din_p_; }
     int dout_pad() const { return dout_p_; }
     unsigned* err_word() const { return err_; }
@@ -79,7 +81,9 @@ class LeafNet {
   private:
     struct Layer;
     void ensure_rows(int rows_pad);
-    void forward(const __nv_bfloat16* x, int rows_pad, float* y, bool keep, cudaStream_t s);
+    // keep: pre-activations kept for backward; h: two buffers for the hidden
+    // activations (null: the layers' own)
+    void forward(const __nv_bfloat16* x, int rows_pad, float* y, bool keep, __nv_bfloat16* const* h, cudaStream_t s);
     // adds the masked mean squared error to *loss (device), leaves the gradients on the device
     void backward(const float* t, const float* mask, int rows_pad, int rows, double* loss, cudaStream_t s);
     void adam(float lr, int step, cudaStream_t s);
@@ -133,6 +137,7 @@ class LeafEvaluator {
     uint16_t* combo_[2] = {nullptr, nullptr};  // hand -> combo
     int16_t* hand_of_[2] = {nullptr, nullptr}; // combo -> hand (-1: none)
     __nv_bfloat16* x_ = nullptr;
+    __nv_bfloat16* h_[2] = {nullptr, nullptr};  // hidden activations
     float* y_ = nullptr;
     float* mass_ = nullptr;  // [row][2]
     float* err_ = nullptr;   // [row]

@@ -92,3 +92,26 @@ def test_trained_network_gains_over_untrained():
         if r["path"] == "full":
             assert r["strategies"] is check.full_strategies
     assert losses["trained"] < 0.5 * losses["untrained"], losses
+
+
+def test_training_with_a_larger_batch_between_iterations():
+    """The network is trained with more rows than the solve's leaves have, after
+    the solve's iteration was captured: the captured products keep their own
+    activations, and the solve goes on with the new weights -- the same, bit for
+    bit, as one whose network was given those weights without being trained."""
+    out = []
+    for trained in (True, False):
+        cfg, spot, host, net, gpu = _dl()
+        gpu.iterate(2)
+        gpu.synchronize()
+        if trained:
+            rng = np.random.default_rng(1)
+            x, t = rng.random((1024, LD.LEAF_IN), np.float32), rng.random((1024, LD.LEAF_OUT), np.float32)
+            net.train(x, t, np.ones_like(t), epochs=1, batch=1024, lr=1e-3, seed=1)
+            weights = [net.params(layer) for layer in range(3)]
+        else:
+            for layer, (w, b) in enumerate(weights):
+                net.set_params(layer, w, b)
+        gpu.iterate(2)
+        out.append([gpu.exploitability(host)] + [gpu.export_arena(k, p) for k in (0, 1) for p in (0, 1)])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
