@@ -403,12 +403,14 @@ struct EngineImpl {
     }
 
     void launch_chance(const Span& sc, int p) {
-        if (!plan.fused) {  // no runout terminals to evaluate in place
+        // the vector and warp engines (no runout terminals in place); the plain
+        // engine, which they are compared with, keeps a kernel of its own
+        if (warp) {
             vec_chance(d, chance + sc.start, sc.count, p, stream);
             return;
         }
-        // runout showdowns: f32 sums in the fused engine, f64 in the plain one
-        if (plan.fused && !term64) k_chance<float><<<sc.count, kThreads, chance_smem, stream>>>(d, chance + sc.start, p);
+        // runout showdowns: f32 sums in the fused32 engine, exact sums else
+        if (!term64) k_chance<float><<<sc.count, kThreads, chance_smem, stream>>>(d, chance + sc.start, p);
         else k_chance<long long><<<sc.count, kThreads, chance_smem, stream>>>(d, chance + sc.start, p);
     }
 
