@@ -32,6 +32,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <future>
 #include <istream>
 #include <map>
 #include <mutex>
@@ -874,6 +875,17 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
     if (E.fmt != kFmtF32 && E.fmt != kFmtI16 && E.fmt != kFmtFP8) throw Error("unknown device arena format");
     if (E.fmt == kFmtFP8 && !staged_kind) throw Error("FP8 arenas run on the staged engine only");
     E.iteration = host.iteration;
+    E.staging_len = std::max<uint64_t>(std::max(sp.tree.data_size[0], sp.tree.data_size[1]), 1);
+    // Pinned memory (read-back chunks only where an arena is worth them) by a
+    // thread of its own beside the plan, which makes no CUDA calls: pinning
+    // 8 MiB takes 4 to 15 ms, the plan of a turn 6.
+    const bool big = E.staging_len * sizeof(float) >= 2 * kPinChunk;
+    int device = 0;
+    CK(cudaGetDevice(&device));
+    std::future<cudaError_t> pinned = std::async([&E, device, big] {
+        const cudaError_t e = cudaSetDevice(device);
+        return e != cudaSuccess ? e : cudaMallocHost(&E.h_dot, 4096 + (big ? 2 * kPinChunk : 0));
+    });
     E.plan = build_plan(sp, host.use_iso, fuse, shard, nshards, leaf_net != nullptr,
                         engine == kEngineStagedRiver && !leaf_net);
     const Plan& P = E.plan;
@@ -1083,11 +1095,8 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
         }
         E.xnodes[q] = dupload(E.hx[q], O, &B, E.stream);
     }
-    E.staging_len = std::max<uint64_t>(std::max(sp.tree.data_size[0], sp.tree.data_size[1]), 1);
     E.staging = (float*)dalloc(E.staging_len * sizeof(float), O, &B, E.stream);
-    // read-back chunks only where an arena is worth them (pinning takes a few ms)
-    const bool big = E.staging_len * sizeof(float) >= 2 * kPinChunk;
-    CK(cudaMallocHost(&E.h_dot, 4096 + (big ? 2 * kPinChunk : 0)));
+    CK(pinned.get());
     if (big) E.pin = (unsigned char*)E.h_dot + 4096;
 
     // upload arenas: quants directly when host and device are both 16-bit, else via f32 (+ encode);

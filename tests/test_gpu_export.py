@@ -27,3 +27,22 @@ def test_first_packed_export_of_a_shard(fmt, algo):
     for which in (0, 1, 2) if algo == "pcfr+" else (0, 1):
         for p in (0, 1):
             np.testing.assert_array_equal(sh.export_arena(which, p), one.export_arena(which, p))
+
+
+def test_engines_read_back_side_by_side():
+    """Seven engines, each read back twice from a thread of its own: every arena
+    as when read back alone."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    hosts = [g.Solver(g.Spot(_flop((0.08 + 0.01 * k, 0.1))), storage="f32", use_iso=False) for k in range(7)]
+    gpus = [g.GpuSolver(h) for h in hosts]
+    for k, gpu in enumerate(gpus):
+        assert hosts[k].spot.data_size[0] * 4 >= 8 << 20
+        gpu.iterate(k + 1)
+    alone = [[gpu.export_arena(1, p) for p in (0, 1)] for gpu in gpus]
+    with ThreadPoolExecutor(7) as pool:
+        for _ in range(2):
+            both = list(pool.map(lambda gpu: [gpu.export_arena(1, p) for p in (0, 1)], gpus))
+            for a, b in zip(alone, both):
+                np.testing.assert_array_equal(a[0], b[0])
+                np.testing.assert_array_equal(a[1], b[1])
