@@ -792,15 +792,16 @@ static void setup_shows(EngineImpl& E) {
     CK(cudaGetLastError());
     auto group = [&](bool upper_only) {
         ShowGroups g = sg;
-        // the level-ordered batches hold one slot each: whole runs move
+        // the level-ordered batches hold one slot each: whole runs move, in parallel
         std::vector<uint32_t> at(P.num_slots + 1, 0);
-        auto each = [&](auto f) {
-            for (size_t l = 0; l < P.show_batch_span.size(); l++) {
-                const Span s = upper_only ? P.show_batch_span_upper[l] : P.show_batch_span[l];
-                for (uint32_t b = s.start; b < s.start + s.count; b++) f(P.show_batch[b]);
+        std::vector<std::pair<uint32_t, uint32_t>> runs;  // (batch, its items' place)
+        for (size_t l = 0; l < P.show_batch_span.size(); l++) {
+            const Span s = upper_only ? P.show_batch_span_upper[l] : P.show_batch_span[l];
+            for (uint32_t b = s.start; b < s.start + s.count; b++) {
+                at[P.show_batch[b].slot + 1] += P.show_batch[b].count;
+                runs.emplace_back(b, 0u);
             }
-        };
-        each([&](const ShowBatch& b) { at[b.slot + 1] += b.count; });
+        }
         const uint32_t G = (uint32_t)g.shape[0].group;
         uint64_t items = 0;
         for (uint32_t s = 0; s < P.num_slots; s++) items += (at[s + 1] + G - 1) / G * G;
@@ -810,9 +811,17 @@ static void setup_shows(EngineImpl& E) {
             for (uint32_t k = n; k < e; k++) it[at[s] + k] = ShowItem{kNoSlot, {0, 0}, s, 0.0f, 0.0f, 0.0f, 0};
             at[s + 1] = at[s] + e;
         }
-        each([&](const ShowBatch& b) {
-            std::copy(P.show.begin() + b.start, P.show.begin() + b.start + b.count, it.begin() + at[b.slot]);
+        for (auto& r : runs) {
+            const ShowBatch& b = P.show_batch[r.first];
+            r.second = at[b.slot];
             at[b.slot] += b.count;
+        }
+        const size_t step = 8192;
+        parallel_for((runs.size() + step - 1) / step, [&](size_t c) {
+            for (size_t k = c * step; k < std::min(runs.size(), (c + 1) * step); k++) {
+                const ShowBatch& b = P.show_batch[runs[k].first];
+                std::copy(P.show.begin() + b.start, P.show.begin() + b.start + b.count, it.begin() + runs[k].second);
+            }
         });
         g.items = dupload(it, O, &B, E.stream);
         g.count = (uint32_t)(items / G);
