@@ -139,7 +139,11 @@ struct EngineImpl {
     XNode* xpacked[2] = {nullptr, nullptr};  // the same blocks packed in order (export of an engine that holds few)
     std::vector<XNode> hx[2];
     void* lock_buf = nullptr;
-    float* staging = nullptr;  // device f32 image of one arena in the reference layout
+    // Device f32 image of one arena in the reference layout.  Between read-backs
+    // it holds the sweep's fold summaries (d.folds), which every sweep writes
+    // before it reads them; everything else that uses it fills what it reads, on
+    // `stream`, and has left it when its call returns.
+    float* staging = nullptr;
     size_t staging_len = 0;
     size_t show_smem = 0;    // plain showdown kernel (f64 scratch)
     size_t act_smem = 0;     // fused up-action dynamic smem
@@ -1010,7 +1014,6 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
             fold_kernels(P.nh[q], fn, &fsm);
             for (const void* f : fn) set_smem(f, fsm);
         }
-        d.folds = (const FoldSum*)dalloc((size_t)E.nfolds * fold_sum_bytes(), O, &B, E.stream);
         auto records = [&](auto KA) {
             constexpr int K = KA();
             PodVec<SNodeT<K>> sn(P.act.size());
@@ -1105,6 +1108,10 @@ GpuEngine::GpuEngine(const HostSolver& host, int fmt, int engine, int shard, int
         E.xnodes[q] = dupload(E.hx[q], O, &B, E.stream);
     }
     E.staging = (float*)dalloc(E.staging_len * sizeof(float), O, &B, E.stream);
+    if (E.vec) {  // a fold's node has at least two actions of a hand: almost always larger than the summary
+        const size_t need = (size_t)E.nfolds * fold_sum_bytes();
+        d.folds = need <= E.staging_len * sizeof(float) ? (const FoldSum*)E.staging : (const FoldSum*)dalloc(need, O, &B, E.stream);
+    }
     CK(pinned.get());
     if (big) E.pin = (unsigned char*)E.h_dot + 4096;
 
@@ -1791,6 +1798,8 @@ void GpuEngine::sync_to_cpu(HostSolver& host, bool strategy_only) {  // gpu/mod.
             const bool whole = !E.plan.iso_active && E.plan.nshards == 1;
             if (E.fmt == kFmtI16 && ha.kind != 0) {
                 // 16-bit on both sides: quants and scales move exactly
+                if (E.plan.visited_action_elems[p] < t.data_size[p])  // nodes the engine does not hold: zeros
+                    CK(cudaMemsetAsync(E.staging, 0, t.data_size[p] * 2, E.stream));
                 k_to_host<uint16_t><<<nb, kThreads, 0, E.stream>>>((const uint16_t*)src, (uint16_t*)E.staging, E.xnodes[p], nh);
                 std::vector<float> sc(E.plan.n_anodes[p]);
                 const float* dsc = which == kRegrets ? E.ar.rscale[p] : which == kStrategy ? E.ar.sscale[p] : E.ar.pscale[p];
@@ -1858,7 +1867,10 @@ uint64_t estimate_vram(const Spot& spot) {  // same role as game.rs:365-373, for
     uint64_t b = P.n_cslots * (uint64_t)P.nh_max * 4 + P.n_rslots[0] * (uint64_t)P.nh[0] * 4 +
                  P.n_rslots[1] * (uint64_t)P.nh[1] * 4;
     b += (P.arena_len[0] + P.arena_len[1]) * 2 * 4;
-    for (const ActItem& a : P.act) b += a.nterm * sizeof(FoldSum);
+    uint64_t folds = 0;  // the fold summaries share the read-back image's memory
+    for (const ActItem& a : P.act) folds += a.nterm * sizeof(FoldSum);
+    const uint64_t image = std::max(spot.tree.data_size[0], spot.tree.data_size[1]) * 4;
+    if (folds > image) b += folds;
     return b + 512ull * 1024 * 1024;
 }
 bool vram_info_mb(uint64_t* free_mb, uint64_t* total_mb) {

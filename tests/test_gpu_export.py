@@ -46,3 +46,51 @@ def test_engines_read_back_side_by_side():
             for a, b in zip(alone, both):
                 np.testing.assert_array_equal(a[0], b[0])
                 np.testing.assert_array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("storage,fmt", [("f32", None), ("compressed", "i16sr"), ("f32", "fp8")])
+def test_read_back_between_iterations(tmp_path, storage, fmt):
+    """The read-back image and the sweeps' fold summaries share memory: an
+    engine read back, synced, saved and queried after every iteration goes on
+    as one that is left alone, bit for bit."""
+    cfg = W.small_flop_spot()
+    ends = []
+    for busy in (True, False):
+        host = g.Solver(g.Spot(cfg), storage=storage)
+        gpu = g.GpuSolver(host, device_format=fmt)
+        for _ in range(4):
+            gpu.iterate(1)
+            if busy:
+                for which in (0, 1):
+                    for p in (0, 1):
+                        gpu.export_arena(which, p)
+                gpu.sync_to_cpu(host)
+                gpu.save(str(tmp_path / "busy.gto"))
+                g.node_strategy(gpu, 0, int(host.spot.tree()["nchild"][0]), int(host.spot.tree()["player"][0]))
+        ends.append([gpu.exploitability()] + [gpu.root_cfv(p, 1) for p in (0, 1)]
+                    + [gpu.export_arena(which, p) for which in (0, 1) for p in (0, 1)])
+    for a, b in zip(*ends):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_sync_of_an_engine_that_holds_few_nodes_leaves_zeros():
+    """A depth-limited solve with 16-bit arenas on both sides: the nodes it does
+    not hold are zeros in the host's arenas, whatever was read back before."""
+    spot = g.Spot(W.flop_spot(g.evaluate7, seed=6, bet=("50",), raise_=(), max_raises=0, pot=100, stack=330,
+                              frac=(0.05, 0.08)))
+    host = g.Solver(spot, storage="compressed", use_iso=False)
+    gpu = g.dl_gpu_solver(host, g.LeafNet(2705, 128, 1, 2652, seed=2), device_format="i16")
+    gpu.iterate(3)
+    for p in (0, 1):
+        gpu.export_arena(1, p)
+    gpu.sync_to_cpu(host)
+    t = spot.tree()
+    visited = g.dl_plan(spot)[3].astype(bool)
+    for p in (0, 1):
+        held = np.zeros(spot.data_size[p], bool)
+        for n in np.nonzero(visited & (t["kind"] == 0) & (t["player"] == p))[0]:
+            held[int(t["data_off"][n]):int(t["data_off"][n]) + int(t["nchild"][n]) * spot.nh[p]] = True
+        for which in (0, 1):
+            a = host.arena(which, p)
+            assert not a[~held].any()
+            np.testing.assert_array_equal(a[held], gpu.export_arena(which, p)[held])
