@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstring>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -30,8 +31,9 @@ struct Events {
             }
     }
 };
-// Chunk j's bytes are moved by `nt` threads, slice by slice; `turn` lets them
-// start on a chunk, `done` counts the slices of each.
+// Chunk j's bytes are moved by `nt` threads, slice by slice (fewer where the
+// system starts no more); `turn` lets them start on a chunk, `done` counts the
+// slices of each.
 struct Crew {
     int nt;
     std::atomic<size_t> turn{0};
@@ -43,17 +45,24 @@ struct Crew {
     }
     template <class F>
     void start(F move) {
-        for (int w = 1; w < nt; w++)
-            ts.emplace_back([this, w, move] {
-                for (size_t j = 0; j < done.size(); j++) {
-                    while (turn.load(std::memory_order_acquire) <= j) {
-                        if (stop.load()) return;
-                        std::this_thread::yield();
-                    }
-                    move(j, w);
-                    done[j].fetch_add(1, std::memory_order_release);
+        auto work = [this, move](int w) {
+            for (size_t j = 0; j < done.size(); j++) {
+                while (turn.load(std::memory_order_acquire) <= j) {
+                    if (stop.load()) return;
+                    std::this_thread::yield();
                 }
-            });
+                move(j, w, nt);
+                done[j].fetch_add(1, std::memory_order_release);
+            }
+        };
+        ts.reserve((size_t)nt);
+        for (int w = 1; w < nt; w++) {
+            try {
+                ts.emplace_back(work, w);
+            } catch (const std::system_error&) {
+                nt = w;  // before the first turn: nobody has read it
+            }
+        }
     }
     void wait(size_t j) const {
         while (done[j].load(std::memory_order_acquire) < nt) std::this_thread::yield();
@@ -74,11 +83,11 @@ void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s, unsi
     }
     const size_t nc = (bytes + kPinChunk - 1) / kPinChunk;
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const int nt = (int)std::min<size_t>(std::min(8u, hw), std::max<size_t>(1, bytes / (kSmall / 2)));
+    const int threads = (int)std::min<size_t>(std::min(8u, hw), std::max<size_t>(1, bytes / (kSmall / 2)));
     Events E;
-    Crew crew(nt, nc);
+    Crew crew(threads, nc);
     auto count = [=](size_t j) { return std::min(kPinChunk, bytes - j * kPinChunk); };
-    auto move = [=](size_t j, int w) {
+    auto move = [=](size_t j, int w, int nt) {
         const size_t n = count(j), pages = (n + 4095) / 4096, per = (pages + nt - 1) / nt * 4096;
         const size_t a = std::min(n, w * per), e = std::min(n, (w + 1) * per);
         std::memcpy((unsigned char*)dst + j * kPinChunk + a, pin + (j & 1) * kPinChunk + a, e - a);
@@ -98,7 +107,7 @@ void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s, unsi
         }
         ck(cudaEventSynchronize(E.ev[j & 1]), "cudaEventSynchronize");
         crew.turn.store(j + 1, std::memory_order_release);
-        move(j, 0);
+        move(j, 0, crew.nt);
         crew.done[j].fetch_add(1, std::memory_order_release);
     }
     for (size_t j = nc > 2 ? nc - 2 : 0; j < nc; j++) crew.wait(j);

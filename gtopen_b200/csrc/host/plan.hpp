@@ -19,6 +19,7 @@
 #include <exception>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 #include <cstdint>
@@ -185,7 +186,14 @@ void parallel_for(size_t n, F f, unsigned max_threads = 16) {
     const unsigned hw = std::thread::hardware_concurrency();
     const size_t nw = std::min<size_t>(n, std::max(1u, std::min({16u, max_threads, hw ? hw : 1u})));
     std::vector<std::thread> ts;
-    for (size_t w = 1; w < nw; w++) ts.emplace_back(work);
+    ts.reserve(nw);
+    for (size_t w = 1; w < nw; w++) {
+        try {
+            ts.emplace_back(work);
+        } catch (const std::system_error&) {
+            break;  // no more threads: those there are take the rest
+        }
+    }
     work();
     for (auto& th : ts) th.join();
     if (err) std::rethrow_exception(err);

@@ -205,13 +205,10 @@ struct EngineImpl {
             const unsigned char* from = d2h_pin[j & 1];
             unsigned char* to = (unsigned char*)dst + off;
             const size_t part = (cnt + nt - 1) / nt;
-            std::vector<std::thread> ts;
-            for (int w = 1; w < nt; w++) {
+            parallel_for((size_t)nt, [&](size_t w) {
                 const size_t a = std::min(cnt, w * part), e = std::min(cnt, a + part);
-                if (a < e) ts.emplace_back([=] { std::memcpy(to + a, from + a, e - a); });
-            }
-            std::memcpy(to, from, std::min(cnt, part));
-            for (auto& t : ts) t.join();
+                std::memcpy(to + a, from + a, e - a);
+            }, (unsigned)nt);
         }
         CK(cudaStreamSynchronize(stream));
     }
@@ -840,21 +837,15 @@ static void setup_shows(EngineImpl& E) {
 // Zeros, by several threads; pages that hold zeros already are only read, so
 // a fresh buffer's pages are not materialised.
 static void zero_fill(void* dst, size_t bytes) {
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int nt = (int)std::max(1u, std::min(8u, hw ? hw : 1u));
-    const size_t pages = (bytes + 4095) / 4096, per = (pages + nt - 1) / nt;
-    auto run = [=](int w) {
-        unsigned char* base = (unsigned char*)dst;
-        for (size_t k = std::min(pages, w * per); k < std::min(pages, (w + 1) * per); k++) {
+    const size_t pages = (bytes + 4095) / 4096, per = 1024;
+    unsigned char* base = (unsigned char*)dst;
+    parallel_for((pages + per - 1) / per, [&](size_t w) {
+        for (size_t k = w * per; k < std::min(pages, (w + 1) * per); k++) {
             unsigned char* q = base + k * 4096;
             const size_t n = std::min<size_t>(4096, bytes - k * 4096);
             if (q[0] != 0 || std::memcmp(q, q + 1, n - 1) != 0) std::memset(q, 0, n);
         }
-    };
-    std::vector<std::thread> ts;
-    for (int w = 1; w < nt; w++) ts.emplace_back(run, w);
-    run(0);
-    for (auto& t : ts) t.join();
+    }, 8);
 }
 
 // --------------------------------------------------------------- GpuEngine
