@@ -14,6 +14,7 @@ namespace gtob {
 
 enum ArenaFormatDev { kDevF32 = 0, kDevI16 = 1, kDevFP8 = 2 };
 
+constexpr unsigned kSms = 148;  // a B200's SMs: the launch thresholds are multiples of it
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxHpt = 6;  // hands per thread in the runout kernel (nh <= 1536)
@@ -77,6 +78,10 @@ struct Arenas {
 };
 
 // ----------------------------------------------------------- small helpers
+// One player's entry of a kernel parameter's pair (a select: an indexed
+// parameter would be copied to local memory).
+template <class T>
+__device__ __forceinline__ T pick(T const (&x)[2], int a) { return a ? x[1] : x[0]; }
 // FP8 E4M3 arena values (the precision-study format): cvt with satfinite --
 // round to nearest even, saturate to +-448 -- and the exact widening back.
 __device__ __forceinline__ uint8_t f32_to_e4m3(float x) {

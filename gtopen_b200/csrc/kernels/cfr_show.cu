@@ -43,9 +43,6 @@
 namespace gtob {
 namespace {
 
-template <class T>
-__device__ __forceinline__ T pick(T const (&x)[2], int a) { return a ? x[1] : x[0]; }
-
 // A board's scan entries: the opponent's hands in strength order (m), then
 // card by card each list of the hands holding the card, in strength order
 // (2 m); bit 15 marks the first entry of the strength order and of each list.
@@ -563,7 +560,7 @@ void vec_folds(const Dev& d, const uint32_t* slots, uint32_t count, int p, cudaS
     const unsigned grid = (count + G - 1) / G, smem = (unsigned)((nho + 3) & ~3) * G * 4;
     FoldSum* out = const_cast<FoldSum*>(d.folds);
     if (G == 32) pdl_launch(kv_folds<32, 1>, grid, fold_threads<32, 1>(), smem, s, d, slots, count, p, out);
-    else if (grid <= 148 * 3) pdl_launch(kv_folds<8, 2>, grid, fold_threads<8, 2>(), smem, s, d, slots, count, p, out);
+    else if (grid <= kSms * 3) pdl_launch(kv_folds<8, 2>, grid, fold_threads<8, 2>(), smem, s, d, slots, count, p, out);
     else pdl_launch(kv_folds<8, 1>, grid, fold_threads<8, 1>(), smem, s, d, slots, count, p, out);
 }
 void vec_chance(const Dev& d, const ChanceItem* items, uint32_t count, int p, cudaStream_t s) {

@@ -392,7 +392,7 @@ __device__ __forceinline__ void ks_down_node(const Dev& d, const Arenas& ar, con
 // The node's fold child, if any, is evaluated here from the staged opponent
 // reach; every other child's cfv is staged from its slot.
 template <int NT = kSThreads>
-struct UpSharedT {  // static shared memory of ks_up (NT threads)
+struct UpSharedT {  // static shared memory of ks_up_node (NT threads)
     int flag;
     long long S[52];
     long long dred[NT / 32];
@@ -938,7 +938,7 @@ __device__ void cta_showdown2(const ShowTab& tb, int nho, int msort, const float
     }
     __syncthreads();
 }
-// Shared memory of ks_show_pair: two barriers, four reach buffers (two
+// Shared memory of show_batch_run: two barriers, four reach buffers (two
 // stages of a pair), the prefix array U (3 msort + 53 pairs), then the slot
 // tables.
 __host__ __device__ inline unsigned show_pair_scratch_bytes(int nh_pad, int msort) {

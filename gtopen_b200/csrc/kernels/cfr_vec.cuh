@@ -52,7 +52,7 @@ namespace {
 // (64 registers: 1.67, 48: 1.64).
 constexpr int kVDownCtas = 16, kVOppCtas = 14, kVMineCtas = 8, kVQuantRegs = 56;
 constexpr int kVMaxWarps = 32;
-constexpr uint64_t kVFillWarps = 148 * 16;  // warps that fill the device
+constexpr uint64_t kVFillWarps = kSms * 16;  // warps that fill the device
 
 // ------------------------------------------------------- register vectors
 template <int B> struct Gran;
@@ -92,11 +92,6 @@ union Pack {
             if (k >= live) e[k] = T(0);
     }
 };
-
-// One player's entry of a kernel parameter's pair (a select: an indexed
-// parameter would be copied to local memory).
-template <class T>
-__device__ __forceinline__ T pick(T const (&x)[2], int a) { return a ? x[1] : x[0]; }
 
 // The thread's place in its node, and the node's scratch in shared memory.
 struct Group {

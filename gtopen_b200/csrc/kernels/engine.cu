@@ -291,11 +291,25 @@ struct EngineImpl {
     // invalidated stream capture.
     void launch_ok(int kind) const {
         const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess)
-            throw Error(std::string("cuda: ") + cudaGetErrorString(e) + " launching a " + kKernelNames[kind] +
-                        " kernel (dynamic shared memory: showdowns " + std::to_string(show_pair_smem) + " B, up " +
-                        std::to_string(st_mine_smem) + "/" + std::to_string(st_opp_smem) + " B, down " +
-                        std::to_string(st_down_smem) + " B)");
+        if (e == cudaSuccess) return;
+        std::string mem;  // the dynamic shared memory of the kernels that take any
+        auto add = [&](const char* what, size_t bytes) {
+            if (bytes) mem += (mem.empty() ? "" : ", ") + std::string(what) + " " + std::to_string(bytes) + " B";
+        };
+        for (int q = 0; vec && q < 2; q++) {
+            const void* fn[2];
+            size_t folds = 0;
+            fold_kernels(plan.nh[q], fn, &folds);
+            if (shows.count) add("showdowns", show_group_smem(shows.shape[q], shows.max_sorted[q], plan.nh[q]));
+            add("folds", folds);
+        }
+        if (!vec) {
+            add("showdowns", show_smem);
+            add("action nodes", warp ? warp_smem : act_smem);
+            add("chance nodes", chance_smem);
+        }
+        throw Error(std::string("cuda: ") + cudaGetErrorString(e) + " launching a " + kKernelNames[kind] +
+                    " kernel (dynamic shared memory: " + (mem.empty() ? "none" : mem) + ")");
     }
     template <class F>
     void timed(Profile* pr, int kind, F launch) {
@@ -425,7 +439,8 @@ struct EngineImpl {
     // 350 v 936 16-bit one 0.293 instead of 0.342, a flop of 28 v 23 hands
     // 0.423 instead of 0.502; one after the other with the dependent launch
     // alone the 16-bit turn takes 0.315.
-    void together(std::initializer_list<std::function<void(cudaStream_t)>> fs) {
+    // kind: what an error of the launches is reported as.
+    void together(int kind, std::initializer_list<std::function<void(cudaStream_t)>> fs) {
         cudaStream_t others[2] = {side, side2};
         cudaEvent_t done[2] = {ev_side, ev_side2};
         if (fs.size() > 1) CK(cudaEventRecord(ev_level, stream));
@@ -441,7 +456,7 @@ struct EngineImpl {
             k++;
         }
         for (int j = 0; j + 1 < k; j++) CK(cudaStreamWaitEvent(stream, done[j], 0));
-        launch_ok(6);
+        launch_ok(kind);
     }
     // One level of the vector kernels' up sweep: the traverser's nodes, the
     // opponent's and the chance nodes read only the level below.
@@ -453,9 +468,9 @@ struct EngineImpl {
         if (mine.count) fs.push_back([&](cudaStream_t st) { vec_up(d, ar, fmt, mine, true, p, eval, st); });
         if (opp.count) fs.push_back([&](cudaStream_t st) { vec_up(d, ar, fmt, opp, false, p, eval, st); });
         if (sc.count) fs.push_back([&](cudaStream_t st) { vec_chance(d, chance + sc.start, sc.count, p, st); });
-        if (fs.size() == 1) together({fs[0]});
-        else if (fs.size() == 2) together({fs[0], fs[1]});
-        else if (fs.size() == 3) together({fs[0], fs[1], fs[2]});
+        if (fs.size() == 1) together(6, {fs[0]});
+        else if (fs.size() == 2) together(6, {fs[0], fs[1]});
+        else if (fs.size() == 3) together(6, {fs[0], fs[1], fs[2]});
     }
     // Down sweep.  qmask: the players whose reach vectors are recomputed.  In a
     // CFR iteration only the opponent's are: the traverser's own reach depends
@@ -473,9 +488,9 @@ struct EngineImpl {
                 const Span sa = plan.act_span_actor[q][l], se = plan.edge_span[l];
                 auto acts = [&](cudaStream_t st) { vec_down(d, ar, fmt, vnodes(sa), d.nh[q], mode, st); };
                 auto edges = [&](cudaStream_t st) { vec_edges(d, edge + se.start, se.count, qmask, st); };
-                if (sa.count && se.count) together({acts, edges});
-                else if (sa.count) together({acts});
-                else if (se.count) together({edges});
+                if (sa.count && se.count) together(1, {acts, edges});
+                else if (sa.count) together(1, {acts});
+                else if (se.count) together(2, {edges});
                 continue;
             }
             if (use_river()) {  // two runs when both players' reach is refreshed
