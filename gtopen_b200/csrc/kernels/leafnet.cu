@@ -80,14 +80,17 @@ __device__ __forceinline__ bool bar_try(uint64_t* b, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-// err: an earlier product's failure ends the wait at once (the products queued
-// behind it would run out their limit one by one); null: the full limit, for
-// what has to finish before a CTA may leave.
+// err: an earlier product's failure ends a wait of over a millisecond (the
+// products queued behind it would run out their limit one by one; a wait of the
+// usual length does not look); null: the full limit, for what has to finish
+// before a CTA may leave.
 __device__ __noinline__ bool bar_wait(uint64_t* b, unsigned parity, const volatile unsigned* err) {
     if (bar_try(b, parity)) return true;
     const unsigned long long t0 = gtimer();
-    while (!bar_try(b, parity))
-        if (gtimer() - t0 > kNetWaitNs || (err && *err)) return false;
+    while (!bar_try(b, parity)) {
+        const unsigned long long t = gtimer() - t0;
+        if (t > kNetWaitNs || (t > 1000000ull && err && *err)) return false;
+    }
     return true;
 }
 __device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -386,8 +389,8 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamLayers
                                               int* applied) {
     __shared__ __nv_bfloat16 t[32][33];
     const int blk = (int)blockIdx.x, c = threadIdx.x & 31, r0 = threadIdx.x >> 5;
-    if (*err) return;
-    if (blk == 0 && threadIdx.x == 0) *applied = step;
+    const bool bad = *err != 0;  // first needed by the stores: on its way beside the loads
+    if (blk == 0 && threadIdx.x == 0 && !bad) *applied = step;
     for (int k = 0; k < A.n; k++) {
         const AdamLayer& L = A.l[k];
         const int tiles = (L.in_p / 32) * (L.out_p / 32);
@@ -401,10 +404,12 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamLayers
                 if (L.live[i]) {
                     float w = L.w[i], m = L.m[i], v = L.v[i];
                     x = __float2bfloat16_rn(adam_one(w, L.g[i], m, v, lr, b1, b2, eps, bc1, bc2));
-                    L.w[i] = w;
-                    L.m[i] = m;
-                    L.v[i] = v;
-                    L.wb[i] = x;
+                    if (!bad) {
+                        L.w[i] = w;
+                        L.m[i] = m;
+                        L.v[i] = v;
+                        L.wb[i] = x;
+                    }
                 }
                 t[r][c] = x;
             }
@@ -412,13 +417,13 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamLayers
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int r = r0 + 8 * j;
-                L.wt[(size_t)(cx + r) * L.out_p + ry + c] = t[c][r];
+                if (!bad) L.wt[(size_t)(cx + r) * L.out_p + ry + c] = t[c][r];
             }
             return;
         }
         if (blk >= L.bias0 && blk < L.bias0 + (L.out + 255) / 256) {
             const int i = (blk - L.bias0) * 256 + (int)threadIdx.x;
-            if (i < L.out) adam_one(L.b[i], L.gb[i], L.mb[i], L.vb[i], lr, b1, b2, eps, bc1, bc2);
+            if (i < L.out && !bad) adam_one(L.b[i], L.gb[i], L.mb[i], L.vb[i], lr, b1, b2, eps, bc1, bc2);
             return;
         }
     }
