@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(NT) kv_show(Dev d, const ShowItem* items, cons
 // vectors serves all of them.  Inside the up kernels these sums took three
 // block barriers and a third of the traverser's instructions per node; as one
 // launch beside the showdowns the opponent's nodes and f32 updates need no
-// barrier at all.  470 v 647 hands, 85,413 folds: 0.13 ms a sweep (issue 74%
-// of peak, the conversions 52%).  One iteration before -> after: that flop,
+// barrier at all.  470 v 647 hands, 85,413 folds: 0.13 and 0.15 ms a sweep (issue
+// 73-75% of peak, 40 registers, 70% of the warps).  One iteration before -> after: that flop,
 // 16-bit, 3.9 -> 3.7 ms; turn f32 0.364 -> 0.291; river f32 0.072 -> 0.058.
 // threads: 52 card lists x 4 lanes (8 folds) x 2 halves of a list, and 26 x 16
 // lanes (32 folds), are 416 -- every thread has a list; a launch that fills
